@@ -122,3 +122,14 @@ def test_io_driven_force():
     g.pp_mean_zx()
     with pytest.raises(ValueError):
         g.driven_force()
+
+
+@pytest.mark.parametrize("thermal", [1, 0])
+@pytest.mark.parametrize("dims", [(8, 4, 8), (22, 5, 10), (64, 6, 8), (66, 7, 18)])
+def test_io_xz_statistics_parity_chunk_edges(dims, thermal):
+    """Rows whose cells fill less than one 64-cell chunk of the reduction, end
+    inside one and end on its boundary."""
+    g, o = _pair(thermal, dims)
+    g.pp_mean_zx()
+    a, _ = g.stats(0)
+    _check_groups(g, a, _oracle_on(g, o, thermal), thermal)
