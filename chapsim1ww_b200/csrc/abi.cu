@@ -561,6 +561,7 @@ static int create_ctx(const chapsim_config *cfg, const chapsim_io_config *iocfg,
     return CHAPSIM_ERR_CUDA;
   }
   ctx->own_stream = ctx->stream;
+  cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device);
   for (auto &e : ctx->ev)
     if (cudaEventCreate(&e) != cudaSuccess) { free_all(ctx); delete ctx; return CHAPSIM_ERR_CUDA; }
   ctx->evpool.assign((size_t)chapsim_ctx::kEvSub * (CHAPSIM_PH_COUNT + 1), nullptr);
@@ -1684,6 +1685,7 @@ int chapsim_set_tuning(chapsim_ctx *ctx, int rhs_nzc, int fft_lb) {
   if (!ctx || rhs_nzc < 1 || fft_lb < 0 || fft_lb > 64 || (fft_lb & 1)) return CHAPSIM_ERR_ARG;
   ctx->rhs_nzc = rhs_nzc;
   ctx->io_nzc = rhs_nzc;  // the IO momentum RHS marches the same way
+  ctx->nzc_set = true;
   ctx->fft_lb = fft_lb;
   drop_graphs(ctx);
   return CHAPSIM_OK;

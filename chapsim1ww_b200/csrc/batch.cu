@@ -65,6 +65,7 @@ int chapsim_batch_create(const chapsim_config *cfgs, int n, chapsim_batch **out)
       delete b;
       return rc;
     }
+    c->batched = true;
     b->ch.push_back(c);
   }
   if (cudaSetDevice(b->device) != cudaSuccess || cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {

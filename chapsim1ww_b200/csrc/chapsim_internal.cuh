@@ -168,6 +168,9 @@ struct chapsim_ctx {
   bool fft_big = false;     // FFT plans with radix 7 or 11
   bool refine = true;       // mixed form: one FP64-residual refinement sweep
   int rhs_nzc = 16;   // z planes per block of k_rhs_tma (autotunable)
+  bool nzc_set = false;  // the caller or the autotuner chose rhs_nzc / io_nzc (else march_len shortens it)
+  bool batched = false;  // a channel of a batch: its kernels share the chip with the other channels'
+  int nsm = 148;      // multiprocessors of the device
   int fft_lb = 0;     // rows per block of the x transforms (0: default)
   int ys_bx = 128;    // spectral y-lines per block of k_ysolve_line (64, 128 or 256; autotunable)
   // IO Poisson with Dirichlet / Neumann x ends (BCX_io): FISHPACK's LP, the
@@ -219,6 +222,20 @@ struct chapsim_ctx {
 
 // Kernel launch wrappers (defined in tg_kernels.cu).
 namespace chapsim {
+// Planes per block of a kernel whose blocks march along z over n planes, one
+// block for each of `tiles` columns: `len`, halved (not below `least`) while
+// there are fewer than `want` blocks.  A short march re-reads more halo
+// planes, so it pays only where the long one leaves multiprocessors without
+// a block, and not in a batch, whose channels fill them together.  Measured
+// on the 64^3 channel, ten steps: 1510 us at 16 and 64 planes for the
+// right-hand side and the x / z factors, 1402 us at 4 and 64, 1398 us at 16
+// and 16, 1300 us at 4 and 16; at 96^3 the factors' march 64 -> 32 gains 3 %
+// and any shorter one of the right-hand side loses.
+inline int march_len(const chapsim_ctx *c, int64_t tiles, int n, int len, int least, int want) {
+  if (c->batched) return len;
+  while (len / 2 >= least && tiles * ((n + len - 1) / len) < want) len /= 2;
+  return len;
+}
 // Phase timer mark: event slot ph of the substep being recorded (timing on).
 inline void phase_mark(chapsim_ctx *c, int ph) {
   if (c->timing) cudaEventRecord(c->evpool[(size_t)c->ev_pending * (CHAPSIM_PH_COUNT + 1) + ph], c->stream);

@@ -1310,6 +1310,12 @@ int io_therm_props(chapsim_ctx *c, int mode) {
   return CHAPSIM_OK;
 }
 
+// z planes per block of k_io_rhs_tma: the caller's choice, or 16, shorter
+// where that gives fewer blocks than multiprocessors
+static int io_march(const chapsim_ctx *c, dim3 grid) {
+  return c->nzc_set ? c->io_nzc : march_len(c, (int64_t)grid.x * grid.y, c->d.nz, c->io_nzc, 4, c->nsm);
+}
+
 int io_mom(chapsim_ctx *c, int ns, bool prep) {
   TGDev &d = c->d;
   IODev &io = c->io;
@@ -1356,12 +1362,13 @@ int io_mom(chapsim_ctx *c, int ns, bool prep) {
   if (c->use_tma_io) {
     IoMaps maps;
     memcpy(maps.m, c->io_maps, sizeof(maps.m));
-    dim3 g2(grid.x, grid.y, (d.nz + c->io_nzc - 1) / c->io_nzc);
+    const int nzc = io_march(c, grid);
+    dim3 g2(grid.x, grid.y, (d.nz + nzc - 1) / nzc);
     constexpr size_t sm = ItGeo<false>::SMEM;
     if (io.thermal)
-      k_io_rhs_tma<true, false><<<g2, blk, sm, c->stream>>>(maps, d, io, sp.gam, sp.roh, sp.alp, cur, c->io_nzc);
+      k_io_rhs_tma<true, false><<<g2, blk, sm, c->stream>>>(maps, d, io, sp.gam, sp.roh, sp.alp, cur, nzc);
     else
-      k_io_rhs_tma<false, false><<<g2, blk, sm, c->stream>>>(maps, d, io, sp.gam, sp.roh, sp.alp, cur, c->io_nzc);
+      k_io_rhs_tma<false, false><<<g2, blk, sm, c->stream>>>(maps, d, io, sp.gam, sp.roh, sp.alp, cur, nzc);
     npart = (int)(g2.x * g2.y * g2.z);
   } else {
     k_io_rhs<<<grid, blk, 0, c->stream>>>(d, io, sp.gam, sp.roh, sp.alp, cur);
@@ -2011,12 +2018,13 @@ int io_np_mom(chapsim_ctx *c, int ns, bool mass_parts) {
   if (c->use_tma_io) {
     IoMaps maps;
     memcpy(maps.m, c->io_maps, sizeof(maps.m));
-    const dim3 g2(grid.x, grid.y, (d.nz + c->io_nzc - 1) / c->io_nzc);
+    const int nzc = io_march(c, grid);
+    const dim3 g2(grid.x, grid.y, (d.nz + nzc - 1) / nzc);
     constexpr size_t sm = ItGeo<true>::SMEM;
     if (io.thermal)
-      k_io_rhs_tma<true, true><<<g2, blk, sm, c->stream>>>(maps, d, io, sp.gam, sp.roh, sp.alp, cur, c->io_nzc);
+      k_io_rhs_tma<true, true><<<g2, blk, sm, c->stream>>>(maps, d, io, sp.gam, sp.roh, sp.alp, cur, nzc);
     else
-      k_io_rhs_tma<false, true><<<g2, blk, sm, c->stream>>>(maps, d, io, sp.gam, sp.roh, sp.alp, cur, c->io_nzc);
+      k_io_rhs_tma<false, true><<<g2, blk, sm, c->stream>>>(maps, d, io, sp.gam, sp.roh, sp.alp, cur, nzc);
   } else {
     k_io_rhs<<<grid, blk, 0, c->stream>>>(d, io, sp.gam, sp.roh, sp.alp, cur);
   }

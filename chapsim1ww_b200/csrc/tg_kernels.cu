@@ -701,7 +701,7 @@ static void launch_adixz(dim3 grid, cudaStream_t st, const TGDev &d, const SubPa
 }
 #undef CHAPSIM_ADIXZ_ROW
 
-constexpr int AR_SEG = 64;  // planes per block of the row form
+constexpr int AR_SEG = 64;  // planes per block of the row form, at most
 // columns per thread of the row form for this nx (0: the tile form runs)
 static int adixz_row_cpt(int nx) {
   if (nx <= 256) return 1;
@@ -709,28 +709,29 @@ static int adixz_row_cpt(int nx) {
   return 0;
 }
 template <typename T, int WX, int WZ, int CPT>
-static void launch_adixz_row_w(dim3 grid, dim3 blk, size_t smem, cudaStream_t st, const TGDev &d,
-                               const SubParams &sp) {
-  k_adixz_row<T, WX, WZ, CPT><<<grid, blk, smem, st>>>(d, sp, AR_SEG);
+static void launch_adixz_row_w(dim3 grid, dim3 blk, size_t smem, cudaStream_t st, const TGDev &d, const SubParams &sp,
+                               int seg) {
+  k_adixz_row<T, WX, WZ, CPT><<<grid, blk, smem, st>>>(d, sp, seg);
 }
 #define CHAPSIM_ADIXZ_RROW(T, WX, CPT)                                                            \
   { launch_adixz_row_w<T, WX, 2, CPT>, launch_adixz_row_w<T, WX, 4, CPT>, launch_adixz_row_w<T, WX, 6, CPT>, \
     launch_adixz_row_w<T, WX, 8, CPT>, launch_adixz_row_w<T, WX, 12, CPT> }
 // the row form of the x / z factors; false when this nx needs the tile form
 template <typename T>
-static bool launch_adixz_rows(cudaStream_t st, const TGDev &d, const SubParams &sp) {
+static bool launch_adixz_rows(cudaStream_t st, const TGDev &d, const SubParams &sp, const chapsim_ctx *c) {
   const int cpt = adixz_row_cpt(d.nx);
   if (!cpt) return false;
-  typedef void (*Fn)(dim3, dim3, size_t, cudaStream_t, const TGDev &, const SubParams &);
+  typedef void (*Fn)(dim3, dim3, size_t, cudaStream_t, const TGDev &, const SubParams &, int);
   static const Fn f1[5][5] = {CHAPSIM_ADIXZ_RROW(T, 2, 1), CHAPSIM_ADIXZ_RROW(T, 4, 1), CHAPSIM_ADIXZ_RROW(T, 6, 1),
                               CHAPSIM_ADIXZ_RROW(T, 8, 1), CHAPSIM_ADIXZ_RROW(T, 12, 1)};
   static const Fn f2[5][5] = {CHAPSIM_ADIXZ_RROW(T, 2, 2), CHAPSIM_ADIXZ_RROW(T, 4, 2), CHAPSIM_ADIXZ_RROW(T, 6, 2),
                               CHAPSIM_ADIXZ_RROW(T, 8, 2), CHAPSIM_ADIXZ_RROW(T, 12, 2)};
   const int iw = band_tw_index(sp.wx), iz = band_tw_index(sp.wz);
   const int btx = d.nx / cpt, bty = btx >= 256 ? 1 : 256 / btx;
-  dim3 blk(btx, bty), grid((d.ny + bty - 1) / bty, 3 * ((d.nz + AR_SEG - 1) / AR_SEG));
+  const int jb = (d.ny + bty - 1) / bty, seg = march_len(c, 3 * jb, d.nz, AR_SEG, 16, c->nsm * 5 / 2);
+  dim3 blk(btx, bty), grid(jb, 3 * ((d.nz + seg - 1) / seg));
   const size_t smem = (size_t)2 * bty * (d.nx + 2 * BAND_TW[iw]) * sizeof(double);
-  (cpt == 1 ? f1 : f2)[iw][iz](grid, blk, smem, st, d, sp);
+  (cpt == 1 ? f1 : f2)[iw][iz](grid, blk, smem, st, d, sp, seg);
   return true;
 }
 #undef CHAPSIM_ADIXZ_RROW
@@ -1629,7 +1630,8 @@ template <typename T> struct Prec {
     {
       dim3 grid((d.nx + RHS_BX - 1) / RHS_BX, (d.ny + RHS_BY - 1) / RHS_BY, d.nz);
       if (c->use_tma_rhs) {
-        const int nzc = c->rhs_nzc;
+        const int nzc =
+            c->nzc_set ? c->rhs_nzc : march_len(c, (int64_t)grid.x * grid.y, d.nz, c->rhs_nzc, 4, c->nsm);
         grid.z = (d.nz + nzc - 1) / nzc;
         RhsMaps maps;
         memcpy(maps.m, c->rhs_maps, sizeof(maps.m));
@@ -1645,7 +1647,7 @@ template <typename T> struct Prec {
     phase_mark(c, CHAPSIM_PH_ADIX);
     if (sp.band) {
       dim3 grid((d.nx + BM_TX - 1) / BM_TX, (d.ny + BM_TY - 1) / BM_TY, 3 * ((d.nz + BM_SEG - 1) / BM_SEG));
-      if (!launch_adixz_rows<T>(c->stream, d, sp)) launch_adixz<T>(grid, c->stream, d, sp);
+      if (!launch_adixz_rows<T>(c->stream, d, sp, c)) launch_adixz<T>(grid, c->stream, d, sp);
       LAUNCHED();
       phase_mark(c, CHAPSIM_PH_ADIZ);
     } else {
