@@ -226,13 +226,11 @@ namespace chapsim {
 // block for each of `tiles` columns: `len`, halved (not below `least`) while
 // there are fewer than `want` blocks.  A short march re-reads more halo
 // planes, so it pays only where the long one leaves multiprocessors without
-// a block, and not in a batch, whose channels fill them together.  Measured
-// on the 64^3 channel, ten steps: 1510 us at 16 and 64 planes for the
+// a block.  Measured on the 64^3 channel, ten steps: 1510 us at 16 and 64 planes for the
 // right-hand side and the x / z factors, 1402 us at 4 and 64, 1398 us at 16
 // and 16, 1300 us at 4 and 16; at 96^3 the factors' march 64 -> 32 gains 3 %
 // and any shorter one of the right-hand side loses.
-inline int march_len(const chapsim_ctx *c, int64_t tiles, int n, int len, int least, int want) {
-  if (c->batched) return len;
+inline int march_len(int64_t tiles, int n, int len, int least, int want) {
   while (len / 2 >= least && tiles * ((n + len - 1) / len) < want) len /= 2;
   return len;
 }

@@ -728,7 +728,9 @@ static bool launch_adixz_rows(cudaStream_t st, const TGDev &d, const SubParams &
                               CHAPSIM_ADIXZ_RROW(T, 8, 2), CHAPSIM_ADIXZ_RROW(T, 12, 2)};
   const int iw = band_tw_index(sp.wx), iz = band_tw_index(sp.wz);
   const int btx = d.nx / cpt, bty = btx >= 256 ? 1 : 256 / btx;
-  const int jb = (d.ny + bty - 1) / bty, seg = march_len(c, 3 * jb, d.nz, AR_SEG, 16, c->nsm * 5 / 2);
+  // the channels of a batch fill the chip together: no shorter marches there
+  const int jb = (d.ny + bty - 1) / bty,
+            seg = c->batched ? AR_SEG : march_len(3 * jb, d.nz, AR_SEG, 16, c->nsm * 5 / 2);
   dim3 blk(btx, bty), grid(jb, 3 * ((d.nz + seg - 1) / seg));
   const size_t smem = (size_t)2 * bty * (d.nx + 2 * BAND_TW[iw]) * sizeof(double);
   (cpt == 1 ? f1 : f2)[iw][iz](grid, blk, smem, st, d, sp, seg);
@@ -1631,7 +1633,7 @@ template <typename T> struct Prec {
       dim3 grid((d.nx + RHS_BX - 1) / RHS_BX, (d.ny + RHS_BY - 1) / RHS_BY, d.nz);
       if (c->use_tma_rhs) {
         const int nzc =
-            c->nzc_set ? c->rhs_nzc : march_len(c, (int64_t)grid.x * grid.y, d.nz, c->rhs_nzc, 4, c->nsm);
+            c->nzc_set ? c->rhs_nzc : march_len((int64_t)grid.x * grid.y, d.nz, c->rhs_nzc, 4, c->nsm);
         grid.z = (d.nz + nzc - 1) / nzc;
         RhsMaps maps;
         memcpy(maps.m, c->rhs_maps, sizeof(maps.m));
