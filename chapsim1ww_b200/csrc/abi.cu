@@ -1283,11 +1283,9 @@ int chapsim_set_table(chapsim_ctx *ctx, const double *H, const double *T, const 
   const double *cols[5] = {H, T, D, M, K};
   for (int q = 0; q < 5; ++q) ctx->tab[q].assign(cols[q], cols[q] + n);
   IODev &io = ctx->io;
-  const std::pair<int, int> xy[4] = {{0, 1}, {1, 2}, {1, 3}, {1, 4}};
-  chapsim_spl::Spline *dst[4] = {&io.ht, &io.td, &io.tm, &io.tk};
-  for (int q = 0; q < 4; ++q) {
-    const cudaError_t e = chapsim_spl::upload_spline(ctx->table_allocs, ctx->tab[xy[q].first], ctx->tab[xy[q].second],
-                                                     *dst[q]);
+  {
+    const cudaError_t e = chapsim_spl::upload_props(ctx->table_allocs, ctx->tab[0], ctx->tab[1], ctx->tab[2],
+                                                    ctx->tab[3], ctx->tab[4], io.tab);
     if (e != cudaSuccess) {
       ctx->err = std::string("property table upload: ") + cudaGetErrorString(e);
       cudaGetLastError();

@@ -62,7 +62,7 @@ struct IODev {
   double *drho;                               // DrhoDtP
   double *rhoh, *h, *T, *D, *D0, *mu, *mu0, *kap, *rhse0;  // RHOH, ENTHALPY, ..., RHS_ENERGY0
   double *msum;                               // mu0 + mu (derived, kept in step)
-  chapsim_spl::Spline ht, td, tm, tk;          // h -> T; T -> rho, mu, k
+  chapsim_spl::PropTable tab;                  // h -> T; T -> rho, mu, k
   double cthecd, qw_bot, qw_top, rhohmax, f_a, cfgv;
   int thermal, shortcuts, gravdir, flowdrvtp;
   // iso-thermal walls: bit 0 bottom, bit 1 top (BCWALLHEAT); wall[side] =

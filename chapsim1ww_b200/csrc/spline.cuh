@@ -44,6 +44,72 @@ __device__ __forceinline__ double spline_at(const Spline &s, int i, double u) {
 }
 __device__ __forceinline__ double spline_eval(const Spline &s, double u) { return spline_at(s, spline_find(s, u), u); }
 
+// ---------------------------------------------------------------- IO tables
+// The table of an IO context, laid out for look-ups by a warp of cells whose
+// enthalpies lie within a hundred or so intervals.  The L1 cache serves a
+// gather one 128-byte line per cycle, so a look-up costs the lines that its
+// gathers touch: coefficients sit in arrays of pairs (a hundred intervals are
+// 13 lines; records of a whole interval are 26 to 100), the search starts
+// from one 4-byte index per bucket, and the caller keeps the last interval's
+// values (Poly), so that a second look-up in it loads nothing.
+struct PropTable {
+  const int *hb, *tb;                 // bucket of the uniform search grid -> first candidate interval
+  const double *hx, *tx;              // the grids of h and T
+  const double2 *hc[2];               // T(h): {c0, c1}, {c2, c3} per interval
+  const double2 *rho[2], *mu[2], *k[2];  // of T
+  double h0, hbinv, t0, tbinv;
+  double hlo, hhi, tlo, thi;
+  int n, nb;
+};
+
+__device__ __forceinline__ bool inside_h(const PropTable &p, double h) { return h > p.hlo && h < p.hhi; }
+__device__ __forceinline__ bool inside_t(const PropTable &p, double T) { return T > p.tlo && T < p.thi; }
+
+// One interval [x, xn) and the coefficients of one function on it:
+// c0 + dx (c1 + dx (c2 + dx c3)), dx = u - x.
+struct Poly {
+  double x, xn;
+  double2 a, b;
+  __device__ __forceinline__ bool holds(double u) const { return u >= x && u < xn; }
+  __device__ __forceinline__ double at(double u) const {
+    const double dx = u - x;
+    return a.x + dx * (a.y + dx * (b.x + dx * b.y));
+  }
+  __device__ __forceinline__ void coef(const double2 *const (&c)[2], int i) {
+    a = __ldg(c[0] + i);
+    b = __ldg(c[1] + i);
+  }
+  // Interval i with x[i] <= u < x[i + 1], u strictly inside the table: from
+  // the bucket's first candidate a few steps up, then by bisection (tables
+  // whose points crowd into few buckets).
+  __device__ __forceinline__ int find(const int *bucket, int nb, double x0, double binv, const double *grid, int n,
+                                      double u) {
+    int q = (int)((u - x0) * binv);
+    q = q < 0 ? 0 : (q >= nb ? nb - 1 : q);
+    int i = __ldg(bucket + q);
+    x = __ldg(grid + i);
+    xn = __ldg(grid + i + 1);
+#pragma unroll 1
+    for (int step = 0; u >= xn; ++step) {
+      if (step == 4) {
+        int j = n - 1;
+        ++i;
+        while (j > i + 1) {
+          const int m = (i + j) >> 1;
+          if (u < __ldg(grid + m)) j = m; else i = m;
+        }
+        x = __ldg(grid + i);
+        xn = __ldg(grid + i + 1);
+        break;
+      }
+      ++i;
+      x = xn;
+      xn = __ldg(grid + i + 1);
+    }
+    return i;
+  }
+};
+
 __device__ __forceinline__ bool inside(const Spline &s, double u) { return u > s.xlo && u < s.xhi; }
 
 
@@ -114,48 +180,62 @@ inline std::vector<int2> bucket_ranges(const std::vector<int> &blo, int n, int n
   return rng;
 }
 
-// Build the spline of y over x on the host and upload x, y, b, c, d, the
-// packed records and the bucket table; every allocation is appended to
-// allocs (freed by the owner).
-inline cudaError_t upload_spline(std::vector<void *> &allocs, const std::vector<double> &x,
-                                 const std::vector<double> &y, Spline &s) {
-  const int n = (int)x.size();
-  std::vector<double> b(n), c(n), d(n);
-  fmm_spline(n, x.data(), y.data(), b.data(), c.data(), d.data());
-  std::vector<int> blo;
-  const int nb = 4 * n;
-  bucket_table(n, x.data(), nb, s.x0, s.binv, blo);
-  void *p = nullptr;
-  cudaError_t e;
-  double *arr[5];
-  const std::vector<double> *src[5] = {&x, &y, &b, &c, &d};
-  for (int q = 0; q < 5; ++q) {
-    if ((e = cudaMalloc(&p, n * sizeof(double))) != cudaSuccess) return e;
-    allocs.push_back(p);
-    arr[q] = (double *)p;
-    if ((e = cudaMemcpy(p, src[q]->data(), n * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
+// First candidate interval of nb uniform buckets: the last one that starts
+// before the bucket, with a margin of 2^-48 of the table's width, far above
+// the rounding of the bucket index.
+inline std::vector<int> first_intervals(int n, const double *x, int nb, double &x0, double &binv) {
+  x0 = x[0];
+  binv = nb / (x[n - 1] - x[0]);
+  const double tol = (x[n - 1] - x[0]) * 0x1p-48;
+  std::vector<int> f(nb);
+  int i = 0;
+  for (int b = 0; b < nb; ++b) {
+    const double start = x0 + b / binv - tol;
+    while (i + 2 < n && x[i + 1] <= start) ++i;
+    f[b] = i;
   }
-  if ((e = cudaMalloc(&p, (nb + 1) * sizeof(int))) != cudaSuccess) return e;
-  allocs.push_back(p);
-  if ((e = cudaMemcpy(p, blo.data(), (nb + 1) * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
-  s.blo = (const int *)p;
-  const std::vector<int2> rng = bucket_ranges(blo, n, nb);
-  if ((e = cudaMalloc(&p, nb * sizeof(int2))) != cudaSuccess) return e;
-  allocs.push_back(p);
-  if ((e = cudaMemcpy(p, rng.data(), nb * sizeof(int2), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
-  s.brng = (const int2 *)p;
-  s.xlo = x[0];
-  s.xhi = x[n - 1];
-  std::vector<double> rec((size_t)4 * n);
-  for (int i = 0; i < n; ++i) { rec[4 * i] = y[i]; rec[4 * i + 1] = b[i]; rec[4 * i + 2] = c[i]; rec[4 * i + 3] = d[i]; }
-  if ((e = cudaMalloc(&p, rec.size() * sizeof(double))) != cudaSuccess) return e;
-  allocs.push_back(p);
-  if ((e = cudaMemcpy(p, rec.data(), rec.size() * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
-  s.ybcd = (const double4 *)p;
-  s.x = arr[0]; s.y = arr[1]; s.b = arr[2]; s.c = arr[3]; s.d = arr[4];
-  s.n = n;
-  s.nb = nb;
-  return cudaSuccess;
+  return f;
+}
+
+// Build the IO table of T(h), rho(T), mu(T), k(T) (FMM splines) on the host
+// and upload it; every allocation is appended to allocs (freed by the owner).
+inline cudaError_t upload_props(std::vector<void *> &allocs, const std::vector<double> &H, const std::vector<double> &T,
+                                const std::vector<double> &D, const std::vector<double> &M,
+                                const std::vector<double> &K, PropTable &p) {
+  const int n = (int)H.size();
+  auto up = [&](const void *src, size_t bytes, const void **dst) {
+    void *q = nullptr;
+    cudaError_t e = cudaMalloc(&q, bytes);
+    if (e != cudaSuccess) return e;
+    allocs.push_back(q);
+    *dst = q;
+    return cudaMemcpy(q, src, bytes, cudaMemcpyHostToDevice);
+  };
+  auto fit = [&](const std::vector<double> &x, const std::vector<double> &y, const double2 *(&c)[2]) {
+    std::vector<double> b(n), cc(n), d(n);
+    fmm_spline(n, x.data(), y.data(), b.data(), cc.data(), d.data());
+    std::vector<double2> lo(n), hi(n);
+    for (int i = 0; i < n; ++i) {
+      lo[i] = make_double2(y[i], b[i]);
+      hi[i] = make_double2(cc[i], d[i]);
+    }
+    const cudaError_t e = up(lo.data(), n * sizeof(double2), (const void **)&c[0]);
+    return e != cudaSuccess ? e : up(hi.data(), n * sizeof(double2), (const void **)&c[1]);
+  };
+  p.n = n;
+  p.nb = 4 * n;
+  const std::vector<int> hb = first_intervals(n, H.data(), p.nb, p.h0, p.hbinv),
+                         tb = first_intervals(n, T.data(), p.nb, p.t0, p.tbinv);
+  p.hlo = H[0]; p.hhi = H[n - 1];
+  p.tlo = T[0]; p.thi = T[n - 1];
+  cudaError_t e;
+  if ((e = fit(H, T, p.hc)) != cudaSuccess || (e = fit(T, D, p.rho)) != cudaSuccess ||
+      (e = fit(T, M, p.mu)) != cudaSuccess || (e = fit(T, K, p.k)) != cudaSuccess)
+    return e;
+  if ((e = up(hb.data(), hb.size() * sizeof(int), (const void **)&p.hb)) != cudaSuccess) return e;
+  if ((e = up(tb.data(), tb.size() * sizeof(int), (const void **)&p.tb)) != cudaSuccess) return e;
+  if ((e = up(H.data(), n * sizeof(double), (const void **)&p.hx)) != cudaSuccess) return e;
+  return up(T.data(), n * sizeof(double), (const void **)&p.tx);
 }
 
 }  // namespace chapsim_spl

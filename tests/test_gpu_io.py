@@ -277,3 +277,36 @@ def test_io_poisson_nonperiodic_x_parity(bcx):
         g.fishpack_pois3d()
         assert relerr(g.get_field("phi"), o.get("phi")) <= 1e-10
         g.close()
+
+
+@pytest.mark.parametrize("n", [8, 37, 300, 4096])
+def test_io_uneven_table_parity(n):
+    """Property look-ups in a table whose points crowd around h = 0 (many of
+    them in one bucket of the look-up's uniform search grid) and are sparse at
+    its ends (many buckets in one interval), against the oracle's binary
+    search; h spread over most of the table."""
+    _need_gpu()
+    from chapsim1ww_b200 import IOChannel
+    from oracle.pyoracle import OracleIO
+    s = np.linspace(-1.0, 1.0, n)
+    H = np.sign(s) * np.abs(s) ** 3 + 0.05 * s
+    T = 1.0 + 0.5 * np.tanh(2.0 * H) + 0.1 * H
+    D = 1.0 / (1.0 + T)
+    M = 0.5 + 0.3 * T * T
+    K = 0.7 + 0.2 * T
+    table = (H, T, D, M, K)
+    dims = (40, 18, 12)
+    g = IOChannel(*dims, thermal=1, table=table)
+    o = OracleIO(*dims, thermal=1, table=table + (np.ones(n),))
+    g.random_fl_theml_fld_io(3, 0.1)
+    o.init_random(3, 0.1)
+    rng = np.random.default_rng(n)
+    h = rng.uniform(-0.95, 0.95, g.shape) * rng.uniform(0.0, 1.0, g.shape) ** 2
+    rhoh = h * o.get("rho")
+    o.set("rhoh", rhoh)
+    g.set_field("rhoh", rhoh)
+    for ns in (1, 2):
+        g.solverrk3_eng_io(ns)
+        o.eng(ns)
+        compare(g, o, THERMAL + ("rho0", "mu0"), tag=f"n {n} eng{ns}")
+    assert g.bad_cells() == o.bad_cells()
