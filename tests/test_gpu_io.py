@@ -310,3 +310,26 @@ def test_io_uneven_table_parity(n):
         o.eng(ns)
         compare(g, o, THERMAL + ("rho0", "mu0"), tag=f"n {n} eng{ns}")
     assert g.bad_cells() == o.bad_cells()
+
+
+@pytest.mark.parametrize("visc", [0, 1])
+def test_io_substep_calls_replay_the_same_launches_bitwise(visc):
+    """Energy and momentum substep calls (captured from the third call of an
+    NS and G buffer on) against graph steps, bitwise, across a change of DT
+    and of the property table."""
+    _need_gpu()
+    from chapsim1ww_b200 import IOChannel
+    from oracle.pyoracle import synth_table
+    a, b = (IOChannel(40, 18, 24, thermal=1, table=synth_table(4096), visc_scheme=visc) for _ in range(2))
+    for x in (a, b):
+        x.random_fl_theml_fld_io(7, 0.1)
+    for change in (lambda x: None, lambda x: x.set_dt(5e-4), lambda x: x.set_table(synth_table(1024))):
+        for x in (a, b):
+            change(x)
+        for _ in range(7):
+            for ns in (1, 2, 3):
+                a.solverrk3_eng_io(ns)
+                a.solverrk3_mom_io(ns)
+        b.step(7)
+        for f in FLOW + THERMAL + ("g0x", "rho0"):
+            assert np.array_equal(a.get_field(f), b.get_field(f)), f

@@ -272,3 +272,26 @@ def test_line_tuning_does_not_change_results():
         res.append([g.get_field(n) for n in ("gx", "p", "h")])
         g.close()
     assert all(np.array_equal(x, y) for x, y in zip(*res))
+
+
+def test_substep_calls_replay_the_same_launches_bitwise():
+    """Substep calls (captured from the third call of an NS on) against graph
+    steps, bitwise, across a change of DT, of the launch shapes and a field
+    written between calls."""
+    _need_gpu()
+    from chapsim1ww_b200 import TGChannel
+    a, b = TGChannel(40, 18, 24), TGChannel(40, 18, 24)
+    for x in (a, b):
+        x.random_fl_fld_tg(7, 0.1)
+    for change in (lambda x: None, lambda x: x.set_dt(5e-4), lambda x: x.set_tuning(8, 4),
+                   lambda x: x.set_field("p", 0.5 * x.get_field("p"))):
+        for x in (a, b):
+            change(x)
+        n0 = a.launch_count(), b.launch_count()
+        for _ in range(4):
+            for ns in (1, 2, 3):
+                a.solverrk3_mom_tg(ns)
+        b.step(4)
+        for f in ("u", "v", "w", "p", "h0u"):
+            assert np.array_equal(a.get_field(f), b.get_field(f)), f
+        assert a.launch_count() - n0[0] == b.launch_count() - n0[1]
