@@ -1343,9 +1343,10 @@ int io_therm_props(chapsim_ctx *c, int mode) {
 }
 
 // z planes per block of k_io_rhs_tma: the caller's choice, or 16, shorter
-// where that gives fewer blocks than multiprocessors
+// where that gives fewer blocks than multiprocessors (not in the mixed form,
+// whose FP32 Poisson solve magnifies the last bits of the mass-flux sum)
 static int io_march(const chapsim_ctx *c, dim3 grid) {
-  return c->nzc_set ? c->io_nzc : march_len((int64_t)grid.x * grid.y, c->d.nz, c->io_nzc, 4, c->nsm);
+  return c->nzc_set || c->cfg.precision == CHAPSIM_MIXED ? c->io_nzc : march_len((int64_t)grid.x * grid.y, c->d.nz, c->io_nzc, 4, c->nsm);
 }
 
 int io_mom(chapsim_ctx *c, int ns, bool prep) {

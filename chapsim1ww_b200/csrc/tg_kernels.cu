@@ -596,84 +596,118 @@ __global__ void __launch_bounds__(BM_TX *BM_TY) k_adixz_band(TGDev d, SubParams 
 }
 
 // Row form of the same factors, used when a block can own whole x rows
-// (nx = CPT * blockDim.x with blockDim.x <= 256): each plane of the block's
-// rows arrives as contiguous rows (no x halo is loaded: the periodic halo is
-// written into shared memory from the row itself), thread tx owns columns
-// tx + c * blockDim.x, c < CPT, and keeps their z windows in registers.
-// Segments of seglen planes per block.
-template <typename T, int WX, int WZ, int CPT>
+// (nx <= 512): thread tx owns the adjacent columns 2 tx, 2 tx + 1 of row ty
+// and keeps their z windows in registers.  Each plane of the block's rows
+// goes through a ring of AR_PD rows in shared memory, every thread copying
+// its own pair with cp.async AR_PD - 1 planes ahead (the register queue of
+// one plane that this replaces kept 10 KB per SM in flight, a third of the
+// DRAM rate); the threads at the row's ends add the periodic halo.  The x
+// band reads 2 + 2 WX values as 16-byte pairs for two results.  One barrier
+// per plane: a slot is refilled after the barrier that follows its last
+// reading.  DPGRNS is subtracted from the x-solved value, times the band's
+// sum; in the mixed form from every value, so that its FP32 Poisson solve,
+// which answers a last-place change of the velocities with 1e-7 of the
+// pressure, sees the same bits as ever.  Segments of seglen planes per block.
+// 256x192x256: 0.207 -> 0.127 ms (FP64), its bytes 0.094 ms.
+constexpr int AR_PD = 6;
+__device__ __forceinline__ void cp_async_pair(double *dst, const double *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_pair(float *dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+template <typename T, int WX, int WZ>
 __global__ void __launch_bounds__(256) k_adixz_row(TGDev d, SubParams sp, int seglen) {
+  typedef typename Cplx<T>::type T2;  // a pair of columns
   constexpr int RS = 2 * WZ + 1;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  double *rows = reinterpret_cast<double *>(smem_raw);  // [2][blockDim.y][nx + 2 WX]
+  T *rows = reinterpret_cast<T *>(smem_raw);  // [AR_PD][blockDim.y][nx + 2 WX]
   const int nx = d.nx, ny = d.ny, nz = d.nz, RW = nx + 2 * WX;
-  const int btx = blockDim.x, tx = threadIdx.x, ty = threadIdx.y;
+  const int tx = threadIdx.x, ty = threadIdx.y, col = 2 * tx;
   const int j = 1 + blockIdx.x * blockDim.y + ty;
   const int comp = blockIdx.y % 3, seg = blockIdx.y / 3;
   const int kb = seg * seglen, ke = min(kb + seglen, nz);
   const bool row_ok = (j <= ny) && !(comp == 1 && j == 1);
-  const double sub = comp == 0 ? d.scal[0] : 0.0;
-  const T *src = reinterpret_cast<const T *>(d.rhs[comp]) + d.sy * (row_ok ? j : 1) + tx;
+  constexpr bool EACH = sizeof(T) == 4;
+  double sub = 0.0;
+  if (comp == 0) {
+    sub = sp.bgx[0];
+#pragma unroll
+    for (int m = 1; m <= WX; ++m) sub += 2.0 * sp.bgx[m];
+    sub = EACH ? d.scal[0] : sub * d.scal[0];
+  }
   // planes [pbeg, pend); the host keeps 2 w + 1 <= nz and WZ <= 2 w, so
   // -nz < pbeg and one wrap per step suffices
   const int pbeg = kb - WZ, pend = ke + WZ;
   const int64_t wrap = d.sz * (int64_t)nz;
-  int lk = pbeg < 0 ? pbeg + nz : pbeg;  // next plane to load
-  const T *lplane = src + d.sz * (int64_t)lk;
-  double na[CPT];
+  int lk = pbeg < 0 ? pbeg + nz : pbeg;  // next plane to copy
+  const T *lplane = reinterpret_cast<const T *>(d.rhs[comp]) + d.sy * (row_ok ? j : 1) + col + d.sz * (int64_t)lk;
+  const int slot_st = blockDim.y * RW;
+  T *const mine = rows + ty * RW + WX + col;
+  int lp = pbeg, lslot = 0;
+  auto copy = [&]() {  // queue plane lp (an empty group past the end)
+    if (row_ok && lp < pend) cp_async_pair(mine + lslot * slot_st, lplane);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    ++lp;
+    lslot = lslot + 1 == AR_PD ? 0 : lslot + 1;
+    lplane += d.sz;
+    if (++lk == nz) { lk = 0; lplane -= wrap; }
+  };
 #pragma unroll
-  for (int c = 0; c < CPT; ++c) na[c] = row_ok ? (double)lplane[c * btx] - sub : 0.0;
-  lplane += d.sz;
-  if (++lk == nz) { lk = 0; lplane -= wrap; }
-  T *dst = reinterpret_cast<T *>(d.dq[comp]) + d.sy * j + tx;
-  double win[CPT][RS];
+  for (int q = 0; q < AR_PD - 1; ++q) copy();
+  T *dst = reinterpret_cast<T *>(d.dq[comp]) + d.sy * j + col;
+  double win[2][RS];
 #pragma unroll
-  for (int c = 0; c < CPT; ++c)
+  for (int c = 0; c < 2; ++c)
 #pragma unroll
     for (int q = 0; q < RS; ++q) win[c][q] = 0.0;
-  int buf = 0;
+  int slot = 0;
   for (int p0 = pbeg; p0 < pend; p0 += RS) {
 #pragma unroll
     for (int u = 0; u < RS; ++u) {
       const int p = p0 + u;
       if (p >= pend) break;  // uniform over the block
-      // publish plane p with its periodic halo (every position of the row
-      // is written for every plane), load plane p + 1.  One barrier per
-      // plane: a buffer is rewritten two planes later.
-      double *row = rows + (size_t)(buf * blockDim.y + ty) * RW;
-      buf ^= 1;
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) {
-        const int col = tx + c * btx;
-        row[col + WX] = na[c];
-        if (col < WX) row[col + nx + WX] = na[c];
-        if (col >= nx - WX) row[col - nx + WX] = na[c];
+      T *row = mine + slot * slot_st;  // this thread's pair of plane p
+      cp_async_wait<AR_PD - 2>();
+      if (row_ok) {
+        // pairs never straddle an end: nx and WX are even
+        if (col < WX) *reinterpret_cast<T2 *>(row + nx) = *reinterpret_cast<const T2 *>(row);
+        if (col >= nx - WX) *reinterpret_cast<T2 *>(row - nx) = *reinterpret_cast<const T2 *>(row);
       }
-      if (row_ok && p + 1 < pend) {
-#pragma unroll
-        for (int c = 0; c < CPT; ++c) na[c] = (double)lplane[c * btx] - sub;
-      }
-      lplane += d.sz;
-      if (++lk == nz) { lk = 0; lplane -= wrap; }
       __syncthreads();
+      copy();
+      slot = slot + 1 == AR_PD ? 0 : slot + 1;
+      double r[2 + 2 * WX];
 #pragma unroll
-      for (int c = 0; c < CPT; ++c) {
-        const double *rr = row + tx + c * btx + WX;
-        double xs = sp.bgx[0] * rr[0];
+      for (int m = 0; m < 2 + 2 * WX; m += 2) {
+        const T2 v = *reinterpret_cast<const T2 *>(row - WX + m);
+        r[m] = EACH ? (double)v.x - sub : (double)v.x;
+        r[m + 1] = EACH ? (double)v.y - sub : (double)v.y;
+      }
 #pragma unroll
-        for (int m = 1; m <= WX; ++m) xs += sp.bgx[m] * (rr[-m] + rr[m]);
-        win[c][u] = xs;
+      for (int c = 0; c < 2; ++c) {
+        double xs = sp.bgx[0] * r[WX + c];
+#pragma unroll
+        for (int m = 1; m <= WX; ++m) xs += sp.bgx[m] * (r[WX + c - m] + r[WX + c + m]);
+        win[c][u] = EACH ? xs : xs - sub;
       }
       if (p - WZ >= kb) {
+        // window planes p - 2 WZ .. p; plane p - t sits in slot (u - t) mod RS
+        T2 o;
+        double acc[2];
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-          // window planes p - 2 WZ .. p; plane p - t sits in slot (u - t) mod RS
-          double acc = sp.bgz[0] * win[c][(u + WZ + 1) % RS];
+        for (int c = 0; c < 2; ++c) {
+          acc[c] = sp.bgz[0] * win[c][(u + WZ + 1) % RS];
 #pragma unroll
           for (int m = 1; m <= WZ; ++m)
-            acc += sp.bgz[m] * (win[c][(u + WZ + 1 - m) % RS] + win[c][(u + WZ + 1 + m) % RS]);
-          if (row_ok) dst[c * btx + d.sz * (int64_t)(p - WZ)] = (T)acc;
+            acc[c] += sp.bgz[m] * (win[c][(u + WZ + 1 - m) % RS] + win[c][(u + WZ + 1 + m) % RS]);
         }
+        o.x = (T)acc[0];
+        o.y = (T)acc[1];
+        if (row_ok) *reinterpret_cast<T2 *>(dst + d.sz * (int64_t)(p - WZ)) = o;
       }
     }
   }
@@ -702,38 +736,34 @@ static void launch_adixz(dim3 grid, cudaStream_t st, const TGDev &d, const SubPa
 #undef CHAPSIM_ADIXZ_ROW
 
 constexpr int AR_SEG = 64;  // planes per block of the row form, at most
-// columns per thread of the row form for this nx (0: the tile form runs)
-static int adixz_row_cpt(int nx) {
-  if (nx <= 256) return 1;
-  if (nx <= 512 && nx % 2 == 0) return 2;
-  return 0;
-}
-template <typename T, int WX, int WZ, int CPT>
+template <typename T, int WX, int WZ>
 static void launch_adixz_row_w(dim3 grid, dim3 blk, size_t smem, cudaStream_t st, const TGDev &d, const SubParams &sp,
                                int seg) {
-  k_adixz_row<T, WX, WZ, CPT><<<grid, blk, smem, st>>>(d, sp, seg);
+  k_adixz_row<T, WX, WZ><<<grid, blk, smem, st>>>(d, sp, seg);
 }
-#define CHAPSIM_ADIXZ_RROW(T, WX, CPT)                                                            \
-  { launch_adixz_row_w<T, WX, 2, CPT>, launch_adixz_row_w<T, WX, 4, CPT>, launch_adixz_row_w<T, WX, 6, CPT>, \
-    launch_adixz_row_w<T, WX, 8, CPT>, launch_adixz_row_w<T, WX, 12, CPT> }
+#define CHAPSIM_ADIXZ_RROW(T, WX)                                                          \
+  { launch_adixz_row_w<T, WX, 2>, launch_adixz_row_w<T, WX, 4>, launch_adixz_row_w<T, WX, 6>, \
+    launch_adixz_row_w<T, WX, 8>, launch_adixz_row_w<T, WX, 12> }
+#define CHAPSIM_ADIXZ_RATTR(T, WX)                                                                   \
+  (const void *)k_adixz_row<T, WX, 2>, (const void *)k_adixz_row<T, WX, 4>, (const void *)k_adixz_row<T, WX, 6>, \
+      (const void *)k_adixz_row<T, WX, 8>, (const void *)k_adixz_row<T, WX, 12>
+static size_t adixz_row_smem(size_t tsize, int rows, int nx, int wx) {
+  return AR_PD * (size_t)rows * (nx + 2 * wx) * tsize;
+}
 // the row form of the x / z factors; false when this nx needs the tile form
 template <typename T>
 static bool launch_adixz_rows(cudaStream_t st, const TGDev &d, const SubParams &sp, const chapsim_ctx *c) {
-  const int cpt = adixz_row_cpt(d.nx);
-  if (!cpt) return false;
+  if (d.nx > 512) return false;
   typedef void (*Fn)(dim3, dim3, size_t, cudaStream_t, const TGDev &, const SubParams &, int);
-  static const Fn f1[5][5] = {CHAPSIM_ADIXZ_RROW(T, 2, 1), CHAPSIM_ADIXZ_RROW(T, 4, 1), CHAPSIM_ADIXZ_RROW(T, 6, 1),
-                              CHAPSIM_ADIXZ_RROW(T, 8, 1), CHAPSIM_ADIXZ_RROW(T, 12, 1)};
-  static const Fn f2[5][5] = {CHAPSIM_ADIXZ_RROW(T, 2, 2), CHAPSIM_ADIXZ_RROW(T, 4, 2), CHAPSIM_ADIXZ_RROW(T, 6, 2),
-                              CHAPSIM_ADIXZ_RROW(T, 8, 2), CHAPSIM_ADIXZ_RROW(T, 12, 2)};
+  static const Fn fns[5][5] = {CHAPSIM_ADIXZ_RROW(T, 2), CHAPSIM_ADIXZ_RROW(T, 4), CHAPSIM_ADIXZ_RROW(T, 6),
+                               CHAPSIM_ADIXZ_RROW(T, 8), CHAPSIM_ADIXZ_RROW(T, 12)};
   const int iw = band_tw_index(sp.wx), iz = band_tw_index(sp.wz);
-  const int btx = d.nx / cpt, bty = btx >= 256 ? 1 : 256 / btx;
+  const int btx = d.nx / 2, bty = 256 / btx;
   // the channels of a batch fill the chip together: no shorter marches there
   const int jb = (d.ny + bty - 1) / bty,
             seg = c->batched ? AR_SEG : march_len(3 * jb, d.nz, AR_SEG, 16, c->nsm * 5 / 2);
   dim3 blk(btx, bty), grid(jb, 3 * ((d.nz + seg - 1) / seg));
-  const size_t smem = (size_t)2 * bty * (d.nx + 2 * BAND_TW[iw]) * sizeof(double);
-  (cpt == 1 ? f1 : f2)[iw][iz](grid, blk, smem, st, d, sp, seg);
+  fns[iw][iz](grid, blk, adixz_row_smem(sizeof(T), bty, d.nx, BAND_TW[iw]), st, d, sp, seg);
   return true;
 }
 #undef CHAPSIM_ADIXZ_RROW
@@ -743,54 +773,114 @@ static bool launch_adixz_rows(cudaStream_t st, const TGDev &d, const SubParams &
 // G[j][m] = (A^{-1})_{j, j+m} for |m| <= WY, precomputed on the host from
 // the Thomas sweeps and truncated where the dropped entries of every row sum
 // to < 2^-60 of its largest entry.  Then q += dq and BC_WALL_Q_tg.  A block
-// owns 32 x-columns, AY_JT rows and one z plane; rows outside [1, ny] carry
-// zero weight.  Per component the block stages its tile of dq (with the y
-// halo) and its AY_JT band rows of G (zero past WY, one zero pad) in shared
-// memory; each thread then computes AY_R consecutive rows of its column,
-// reading each tile value once and the band coefficients as 16-byte
-// broadcast pairs.  W is a compile-time width at least WY.  The v line's
-// row-1 right-hand side is the final u increment at j = 1 (the reference
-// quirk described at k_adiy_smem), computed here from the u data.
+// owns 32 x-columns, AY_JT rows, one component and a segment of z planes;
+// rows outside [1, ny] carry zero weight.  It stages its AY_JT band rows of G
+// (zero past WY, one zero pad) once and marches over its planes: the tiles of
+// dq (with the y halo) go through a ring of AY_PD tiles in shared memory,
+// copied with cp.async AY_PD - 1 planes ahead, and the q of plane k + 1 is
+// loaded into registers while plane k is computed, so that one barrier per
+// plane suffices and no load is waited for.  Each thread computes AY_R
+// consecutive rows of its column, reading each tile value once and the band
+// coefficients as 16-byte broadcast pairs.  W is a compile-time width at
+// least WY.  The v line's row-1 right-hand side is the final u increment at
+// j = 1 (the reference quirk described at k_adiy_smem), computed here from
+// the u data.  256x192x256: 0.260 -> 0.200 ms, its bytes 0.140 ms (one plane
+// and all three components per block, every load waited for at a barrier,
+// before; with the next tile in registers 0.219 ms).
 constexpr int AY_JT = 32, AY_TX = 32, AY_TY = 8, AYB_WMAX = 16, AY_R = AY_JT / AY_TY;
 constexpr int AY_TW[6] = {2, 4, 6, 8, 12, 16};  // compiled widths
+constexpr int AY_SEG = 16;                      // planes per block, at most
+constexpr int AY_PD = 4;                        // tiles of the ring
 static_assert(AY_TW[5] == AYB_WMAX, "the widest compiled band is the host's limit");
 template <typename T, int W>
-__global__ void __launch_bounds__(AY_TX *AY_TY) k_adiy_band(TGDev d, SubParams sp) {
+__global__ void __launch_bounds__(AY_TX *AY_TY) k_adiy_band(TGDev d, SubParams sp, int seg) {
   constexpr int NT = AY_R + 2 * W + 1;  // tile values per thread; the last one meets a zero weight
   constexpr int GS = 2 * W + 2;         // band row stride in shared memory (even: pairs stay 16-byte aligned)
-  __shared__ double tile[(AY_JT + 2 * W + 1) * AY_TX];
+  constexpr int NR = AY_JT + 2 * W;     // tile rows j0-W .. j0+AY_JT-1+W, then one zero row
+  constexpr int TS = (NR + 1) * AY_TX;  // one tile
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  T *ring = reinterpret_cast<T *>(smem_raw);
   __shared__ __align__(16) double gsh[AY_JT * GS];
-  __shared__ double du1[AY_TX];
+  constexpr bool APART = sizeof(T) == 4;  // row 1 of the v lines is FP64 in the mixed form too: beside the FP32 tile
+  __shared__ double vrow[2][AY_TX];
   const int nx = d.nx, ny = d.ny;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + AY_TX * ty;
-  const int x0 = blockIdx.x * AY_TX, j0 = 1 + blockIdx.y * AY_JT, k = blockIdx.z;
+  const int x0 = blockIdx.x * AY_TX, j0 = 1 + blockIdx.y * AY_JT, comp = blockIdx.z % 3;
+  const int kb = blockIdx.z / 3 * seg, ke = min(kb + seg, d.nz);
   const int i = x0 + tx;
   const bool col_ok = i < nx;
-  const int64_t base = (int64_t)i + d.sz * k;
-  const int nrow = AY_JT + 2 * W;  // tile rows j0-W .. j0+AY_JT-1+W, then one zero row
-  const int jr0 = ty * AY_R;
-  for (int comp = 0; comp < 3; ++comp) {
-    const T *src = reinterpret_cast<const T *>(d.dq[comp]);
-    for (int r = ty; r <= nrow; r += AY_TY) {
-      const int j = j0 - W + r;
-      double v = 0.0;
-      if (col_ok && r < nrow && j >= 1 && j <= ny) v = (double)src[base + d.sy * j];
-      tile[r * AY_TX + tx] = v;
+  const int jr0 = ty * AY_R, jlo = comp == 1 ? 2 : 1;
+  const bool row1 = comp == 1 && j0 == 1;  // the block computes row 1 of the v lines itself
+  // copies: 16 lanes per row, a pair of columns each (nx even: a pair is
+  // inside or outside the field)
+  const int cc = 2 * (tid & 15), cr = tid >> 4;
+  const T *src = reinterpret_cast<const T *>(d.dq[comp]) + x0 + cc + d.sz * kb + d.sy * (j0 - W);
+  const T *su = reinterpret_cast<const T *>(d.dq[0]) + i + d.sz * kb + d.sy;
+  double *q = (comp == 0 ? d.u : (comp == 1 ? d.v : d.w)) + i + d.sz * kb;
+  for (int t = tid; t < AY_JT * GS; t += AY_TX * AY_TY) {
+    // band rows G[j][m], m = -W .. W + 1 (the last zero); rows past ny repeat
+    // row ny and are discarded
+    const int r = t / GS, m = t - r * GS - W, j = min(j0 + r, ny);
+    gsh[t] = m <= W ? sp.yg[comp][(size_t)j * (2 * AYB_WMAX + 1) + AYB_WMAX + m] : 0.0;
+  }
+  // rows that no copy fills stay zero
+  for (int t = tid; t < AY_PD * TS; t += AY_TX * AY_TY) {
+    const int row = t % TS / AY_TX, j = j0 - W + row;
+    if (row == NR || j < 1 || j > ny || (row1 && row == W)) ring[t] = (T)0;
+  }
+  int kc = kb, cslot = 0;
+  auto copy = [&]() {  // queue plane kc (an empty group past the end)
+    if (kc < ke && x0 + cc < nx) {
+      T *t = ring + cslot * TS + cc;
+#pragma unroll
+      for (int r = 0; r < (NR + 15) / 16; ++r) {
+        const int row = cr + 16 * r, j = j0 - W + row;
+        if (row < NR && j >= 1 && j <= ny && !(row1 && row == W)) cp_async_pair(t + row * AY_TX, src + d.sy * row);
+      }
     }
-    // the block's band rows G[j][m], m = -W .. W + 1 (the last zero); rows
-    // past ny repeat row ny and are discarded
-    const double *G = sp.yg[comp];
-    for (int t = tid; t < AY_JT * GS; t += AY_TX * AY_TY) {
-      const int r = t / GS, m = t - r * GS - W, j = min(j0 + r, ny);
-      gsh[t] = m <= W ? G[(size_t)j * (2 * AYB_WMAX + 1) + AYB_WMAX + m] : 0.0;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    ++kc;
+    cslot = cslot + 1 == AY_PD ? 0 : cslot + 1;
+    src += d.sz;
+  };
+  double nq[AY_R];
+  double v1 = 0.0;  // row j = 1 of the v lines
+  auto load = [&]() {
+#pragma unroll
+    for (int r = 0; r < AY_R; ++r) {
+      const int j = j0 + jr0 + r;
+      nq[r] = (col_ok && j >= jlo && j <= ny) ? q[d.sy * j] : 0.0;
     }
-    if (comp == 1 && j0 == 1) {
-      __syncthreads();
-      if (ty == 0) tile[(1 - j0 + W) * AY_TX + tx] = du1[tx];  // row j = 1 of v <- u increment
+    if (row1 && ty == 0 && col_ok) {
+      // the u increment at j = 1, the same sum as the u block's
+      const double *G = sp.yg[0] + (2 * AYB_WMAX + 1) + AYB_WMAX;
+      v1 = 0.0;
+#pragma unroll
+      for (int m = 0; m <= W; ++m)
+        if (m < ny) v1 += G[m] * (double)su[d.sy * m];
     }
+  };
+#pragma unroll
+  for (int r = 0; r < AY_PD - 1; ++r) copy();
+  load();
+  int slot = 0;
+  for (int k = kb; k < ke; ++k) {
+    T *tl = ring + slot * TS;
+    const int vs = (k - kb) & 1;
+    cp_async_wait<AY_PD - 2>();
+    if (row1 && ty == 0) {
+      if (APART) vrow[vs][tx] = v1; else tl[W * AY_TX + tx] = (T)v1;
+    }
+    double old[AY_R];
+#pragma unroll
+    for (int r = 0; r < AY_R; ++r) old[r] = nq[r];
+    double *qk = q;
     __syncthreads();
-    double *q = comp == 0 ? d.u : (comp == 1 ? d.v : d.w);
-    const int jlo = comp == 1 ? 2 : 1;
+    copy();
+    slot = slot + 1 == AY_PD ? 0 : slot + 1;
+    su += d.sz;
+    q += d.sz;
+    if (k + 1 < ke) load();
     double acc[AY_R];
     double2 cp[AY_R];
 #pragma unroll
@@ -801,7 +891,8 @@ __global__ void __launch_bounds__(AY_TX *AY_TY) k_adiy_band(TGDev d, SubParams s
     // tile row jr0 + qq feeds row r with the weight G[j0 + jr0 + r][qq - r - W]
 #pragma unroll
     for (int qq = 0; qq < NT; ++qq) {
-      const double v = tile[(jr0 + qq) * AY_TX + tx];
+      double v = (double)tl[(jr0 + qq) * AY_TX + tx];
+      if (APART && row1 && jr0 + qq == W) v = vrow[vs][tx];
 #pragma unroll
       for (int r = 0; r < AY_R; ++r) {
         const int m2 = qq - r;  // m + W
@@ -813,33 +904,34 @@ __global__ void __launch_bounds__(AY_TX *AY_TY) k_adiy_band(TGDev d, SubParams s
 #pragma unroll
     for (int r = 0; r < AY_R; ++r) {
       const int j = j0 + jr0 + r;
-      if (j > ny) break;  // uniform over the warp (one warp per ty)
-      if (comp == 0 && j == 1) du1[tx] = acc[r];
-      if (col_ok && j >= jlo) q[base + d.sy * j] += acc[r];
+      if (col_ok && j >= jlo && j <= ny) qk[d.sy * j] = old[r] + acc[r];
     }
     if (col_ok && ty == 0) {
       if (j0 == 1) {
-        q[base] = 0.0;
-        if (comp == 1) q[base + d.sy] = 0.0;
+        qk[0] = 0.0;
+        if (comp == 1) qk[d.sy] = 0.0;
       }
-      if (j0 + AY_JT > ny) q[base + d.sy * (ny + 1)] = 0.0;
+      if (j0 + AY_JT > ny) qk[d.sy * (ny + 1)] = 0.0;
     }
-    __syncthreads();
   }
 }
+static size_t adiy_ring_smem(size_t tsize, int w) { return AY_PD * (size_t)(AY_JT + 2 * w + 1) * AY_TX * tsize; }
 template <typename T, int W>
-static void launch_adiy_w(dim3 grid, cudaStream_t st, const TGDev &d, const SubParams &sp) {
-  k_adiy_band<T, W><<<grid, dim3(AY_TX, AY_TY), 0, st>>>(d, sp);
+static void launch_adiy_w(dim3 grid, cudaStream_t st, const TGDev &d, const SubParams &sp, int seg) {
+  k_adiy_band<T, W><<<grid, dim3(AY_TX, AY_TY), adiy_ring_smem(sizeof(T), W), st>>>(d, sp, seg);
 }
 // the band form of the y factors (the host keeps 0 <= wy <= AYB_WMAX when it is on)
 template <typename T>
-static void launch_adiy(dim3 grid, cudaStream_t st, const TGDev &d, const SubParams &sp) {
-  typedef void (*Fn)(dim3, cudaStream_t, const TGDev &, const SubParams &);
+static void launch_adiy(const chapsim_ctx *c, const TGDev &d, const SubParams &sp) {
+  typedef void (*Fn)(dim3, cudaStream_t, const TGDev &, const SubParams &, int);
   static const Fn fns[6] = {launch_adiy_w<T, 2>, launch_adiy_w<T, 4>, launch_adiy_w<T, 6>,
                             launch_adiy_w<T, 8>, launch_adiy_w<T, 12>, launch_adiy_w<T, 16>};
   int q = 0;
   while (q < 5 && sp.wy > AY_TW[q]) ++q;
-  fns[q](grid, st, d, sp);
+  dim3 grid((d.nx + AY_TX - 1) / AY_TX, (d.ny + AY_JT - 1) / AY_JT, 1);
+  const int seg = march_len((int64_t)3 * grid.x * grid.y, d.nz, AY_SEG, 2, 3 * c->nsm);
+  grid.z = 3 * ((d.nz + seg - 1) / seg);
+  fns[q](grid, c->stream, d, sp, seg);
 }
 
 // ============================================================ y lines
@@ -1541,6 +1633,15 @@ template <typename T> struct Prec {
                          (const void *)k_fftx<T, false>,  (const void *)k_ifftx<T, false>,   (const void *)k_fftz<T, false>,
                          (const void *)k_fftx<T, true>,   (const void *)k_ifftx<T, true>,    (const void *)k_fftz<T, true>,
                          (const void *)k_adiy_smem<T>};
+    const void *row[] = {CHAPSIM_ADIXZ_RATTR(T, 2), CHAPSIM_ADIXZ_RATTR(T, 4), CHAPSIM_ADIXZ_RATTR(T, 6),
+                         CHAPSIM_ADIXZ_RATTR(T, 8), CHAPSIM_ADIXZ_RATTR(T, 12)};
+    // rows of short lines with wide halos: 64 rows of 8 + 24 values, 98 KB
+    for (const void *f : row) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    const void *yband[] = {(const void *)k_adiy_band<T, 2>, (const void *)k_adiy_band<T, 4>,
+                           (const void *)k_adiy_band<T, 6>, (const void *)k_adiy_band<T, 8>,
+                           (const void *)k_adiy_band<T, 12>, (const void *)k_adiy_band<T, 16>};
+    for (const void *f : yband)
+      CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adiy_ring_smem(sizeof(T), AYB_WMAX)));
     for (const void *f : dyn) {
       cudaFuncAttributes fa;
       CK(cudaFuncGetAttributes(&fa, f));
@@ -1632,8 +1733,11 @@ template <typename T> struct Prec {
     {
       dim3 grid((d.nx + RHS_BX - 1) / RHS_BX, (d.ny + RHS_BY - 1) / RHS_BY, d.nz);
       if (c->use_tma_rhs) {
-        const int nzc =
-            c->nzc_set ? c->rhs_nzc : march_len((int64_t)grid.x * grid.y, d.nz, c->rhs_nzc, 4, c->nsm);
+        // (the mixed form keeps its block order, and with it the bits of the
+        // mass-flux sum: its FP32 Poisson solve magnifies them)
+        const int nzc = c->nzc_set || sizeof(T) == 4
+                            ? c->rhs_nzc
+                            : march_len((int64_t)grid.x * grid.y, d.nz, c->rhs_nzc, 4, c->nsm);
         grid.z = (d.nz + nzc - 1) / nzc;
         RhsMaps maps;
         memcpy(maps.m, c->rhs_maps, sizeof(maps.m));
@@ -1664,8 +1768,7 @@ template <typename T> struct Prec {
     }
     phase_mark(c, CHAPSIM_PH_ADIY);
     if (sp.band && sp.wy >= 0) {
-      dim3 grid((d.nx + AY_TX - 1) / AY_TX, (d.ny + AY_JT - 1) / AY_JT, d.nz);
-      launch_adiy<T>(grid, c->stream, d, sp);
+      launch_adiy<T>(c, d, sp);
       LAUNCHED();
     } else {
       dim3 grid((d.nx + AY_TL - 1) / AY_TL, d.nz);

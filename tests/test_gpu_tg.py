@@ -295,3 +295,26 @@ def test_substep_calls_replay_the_same_launches_bitwise():
         for f in ("u", "v", "w", "p", "h0u"):
             assert np.array_equal(a.get_field(f), b.get_field(f)), f
         assert a.launch_count() - n0[0] == b.launch_count() - n0[1]
+
+
+@pytest.mark.parametrize("dims", [(8, 4, 8), (10, 33, 66), (30, 65, 18), (512, 5, 16), (528, 6, 20)])
+def test_adi_factor_edges(dims):
+    """The x / z and y factors at the ends of their shapes: the shortest and
+    longest rows of the row form and the first of the tile form (nx 512, 528),
+    one row past a y tile, plane counts that leave short last segments and
+    fewer planes than the copies run ahead."""
+    g, o = pair(*dims, seed=4)
+    for ns in (0, 1, 2, 3):
+        g.solverrk3_mom_tg(ns)
+        o.substep(ns)
+        compare(g, o, tag=f"ns{ns}")
+
+
+@pytest.mark.parametrize("dt,ren", [(5e-3, 200.0), (1e-2, 100.0), (2e-2, 100.0)])
+def test_adi_factor_wider_bands(dt, ren):
+    """Wider compiled bands of the factors (larger dt / Re)."""
+    g, o = pair(40, 36, 24, ren=ren, dt=dt, seed=4)
+    for ns in (0, 1, 2, 3):
+        g.solverrk3_mom_tg(ns)
+        o.substep(ns)
+        compare(g, o, tag=f"ns{ns}")
