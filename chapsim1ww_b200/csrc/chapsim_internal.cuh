@@ -17,11 +17,15 @@ namespace chapsim {
 // Device-side parameters of one TG domain, passed by value to every kernel.
 // Index convention: field(i, j, k) at i + nx*(j + (ny+2)*k), i in [0,nx),
 // j in [0,ny+1] (j = 0 and ny+1 are the wall ghost layers), k in [0,nz).
-// Spectral data: S(kx, j, kz) at kx + lp*((j-1) + ny*kz), kx in [0,lh).
+// Spectral data: S(kx, j, kz) at kx + lp*(kz + nz*(j-1)), kx in [0,lh): the z
+// transform of a row j stays within lp*nz consecutive values.
 struct TGDev {
   int nx, ny, nz, lh;
   int lp;          // pitch of a spectral row: lh rounded up to even (16-byte rows)
   int64_t sy, sz;  // strides of j and k in a field
+  // first value of spectral row (j, kz), j in [1, ny], and the stride of j
+  __host__ __device__ int64_t srow(int j, int kz) const { return (int64_t)lp * (kz + (int64_t)nz * (j - 1)); }
+  __host__ __device__ int64_t ssj() const { return (int64_t)lp * nz; }
   // FP64 state
   double *u, *v, *w, *p, *phi, *rhsphi;
   void *h0[3];      // CONVH0 (temporary precision)
@@ -130,6 +134,14 @@ struct FFTPlan {
   const float2 *tw32;
 };
 
+// Stages of a register-blocked line (fft_reg.cuh): nst radices, the largest in
+// rmax; no plan when nst = 0.
+struct RegPlan {
+  int n, nst, rmax;
+  int R[3];
+  const double2 *tw;  // exp(-2 pi i m / n), filled in at each launch
+};
+
 }  // namespace chapsim
 
 struct chapsim_ctx {
@@ -141,6 +153,7 @@ struct chapsim_ctx {
 
   chapsim::TGDev d{};
   chapsim::FFTPlan fx{}, fz{};
+  chapsim::RegPlan rz{};  // the z transform's register-blocked stages (none: nst = 0)
   // host mesh copies
   std::vector<double> ynd, ycc, dyfi, dyci, wff, wfb;
   double area_inlet = 0.0;

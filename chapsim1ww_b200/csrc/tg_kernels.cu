@@ -22,6 +22,7 @@
 #include <string.h>
 
 #include "chapsim_internal.cuh"
+#include "fft_reg.cuh"
 #include "fft_smem.cuh"
 #include "tma.cuh"
 
@@ -1098,8 +1099,8 @@ __global__ void __launch_bounds__(256, BIG ? 2 : 3) k_fftx(TGDev d, SubParams sp
     x1.x = (T)0.5 * (z.y - zc.y) * scale;
     x1.y = (T)-0.5 * (z.x - zc.x) * scale;
     const int r0 = 2 * p;
-    if (r0 < nrow) S[kx + (int64_t)d.lp * ((jbeg + r0 - 1) + (int64_t)ny * k)] = x0;
-    if (r0 + 1 < nrow) S[kx + (int64_t)d.lp * ((jbeg + r0) + (int64_t)ny * k)] = x1;
+    if (r0 < nrow) S[kx + d.srow(jbeg + r0, k)] = x0;
+    if (r0 + 1 < nrow) S[kx + d.srow(jbeg + r0 + 1, k)] = x1;
   }
 }
 
@@ -1115,7 +1116,7 @@ __global__ void __launch_bounds__(256, BIG ? 2 : 3) k_fftz(TGDev d, FFTPlan pl, 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint64_t bar;
   __shared__ int rad[16];
-  const int nz = d.nz, ny = d.ny, lh = d.lh;
+  const int nz = d.nz, lh = d.lh;
   const int j = blockIdx.y + 1;
   const int kx0 = blockIdx.x * lz;
   const int nl = min(lz, lh - kx0);
@@ -1131,8 +1132,8 @@ __global__ void __launch_bounds__(256, BIG ? 2 : 3) k_fftz(TGDev d, FFTPlan pl, 
   }
   if (tid < 16) rad[tid] = pl.rad[tid];
   __syncthreads();
-  C *S = reinterpret_cast<C *>(d.spec) + kx0 + (int64_t)d.lp * (j - 1);
-  const int64_t skz = (int64_t)d.lp * ny;
+  C *S = reinterpret_cast<C *>(d.spec) + kx0 + d.srow(j, 0);
+  const int64_t skz = d.lp;
   const uint32_t rowb = (uint32_t)(nc * sizeof(C));
   if (tid == 0) mbar_expect_tx(&bar, rowb * (uint32_t)nz);
   __syncthreads();
@@ -1166,6 +1167,81 @@ __global__ void __launch_bounds__(256, BIG ? 2 : 3) k_fftz(TGDev d, FFTPlan pl, 
   }
 }
 
+// The z transform of FP64 spectra with register-blocked lines (fft_reg.cuh):
+// thread (l, j) of a block's lz lines (consecutive kx) takes butterfly j of
+// line l in every stage, its points straight from global memory in the first
+// and its results straight to it from the last, so that 256 points cross
+// shared memory once instead of four times (staging and three radix-8
+// stages).  The scale and the zeroed mean mode are those of k_fftz.  Forward /
+// inverse, against k_fftz: 72 / 68 -> 67 / 58 us at 256x192x256, 88 / 86 ->
+// 72 / 64 at 384x192x192, 49 / 47 -> 25 / 21 at 210x99x154 (no integer
+// divisions at lengths that are not powers of two), then 66 / 56, 70 / 62 and
+// 24 / 21 with the rows of one j consecutive in memory.  Bound by the latency
+// of its strided row reads at 16 warps per SM.
+template <int RMAX, int SG>
+__global__ void __launch_bounds__(256, RMAX > 8 ? 2 : 3) k_fftz_reg(TGDev d, RegPlan pl, int llz) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  double2 *A = reinterpret_cast<double2 *>(smem_raw);  // A[e * lz + l]
+  const int n = pl.n, lz = 1 << llz, l = threadIdx.x & (lz - 1), j = threadIdx.x >> llz;
+  const int row = blockIdx.y, kx = blockIdx.x * lz + l;
+  const bool line = kx < d.lh;
+  const int64_t skz = d.lp;
+  double2 *S = reinterpret_cast<double2 *>(d.spec) + kx + d.srow(row + 1, 0);
+  with_radix<RMAX>(pl.R[0], [&](auto tag) {
+    constexpr int R = decltype(tag)::value;
+    const int nb = n / R;
+    if (j < nb && line) {
+      double2 v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = S[skz * (j + r * nb)];
+      Dft<R, SG>::run(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) A[((j * R + r) << llz) + l] = v[r];
+    }
+  });
+  __syncthreads();
+  int Ns = pl.R[0];
+  if (pl.nst == 3) {
+    with_radix<RMAX>(pl.R[1], [&](auto tag) {
+      constexpr int R = decltype(tag)::value;
+      const int nb = n / R, jq = j / Ns, k = j - jq * Ns;
+      double2 v[R];
+      if (j < nb && line) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = A[((j + r * nb) << llz) + l];
+        reg_twiddle<R, SG>(v, pl.tw, k * (n / (Ns * R)));
+        Dft<R, SG>::run(v);
+      }
+      __syncthreads();
+      if (j < nb && line) {
+        const int base = jq * Ns * R + k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) A[((base + r * Ns) << llz) + l] = v[r];
+      }
+    });
+    __syncthreads();
+    Ns *= pl.R[1];
+  }
+  with_radix<RMAX>(pl.nst == 3 ? pl.R[2] : pl.R[1], [&](auto tag) {
+    constexpr int R = decltype(tag)::value;
+    const int nb = n / R;  // = Ns
+    if (j < nb && line) {
+      double2 v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = A[((j + r * nb) << llz) + l];
+      reg_twiddle<R, SG>(v, pl.tw, j);
+      Dft<R, SG>::run(v);
+      const double scale = SG < 0 ? 1.0 / n : 1.0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        double2 x = make_double2(v[r].x * scale, v[r].y * scale);
+        if (SG < 0 && r == 0 && j == 0 && row == 0 && kx == 0 && !d.pin_last) x = make_double2(0.0, 0.0);
+        S[skz * (j + r * nb)] = x;
+      }
+    }
+  });
+}
+
 // Pivots of the Poisson y-tridiagonals, computed once per context: for every
 // (kx, kz) the forward-elimination factors pp_j = 1/(B_j - h_{j-1} A_j) and
 // h_j = C_j pp_j of the matrix of src/possion3d_FFT99.f90:334-443 with the
@@ -1178,7 +1254,7 @@ __global__ void k_ypivots(TGDev d) {
   const int kx = blockIdx.x * blockDim.x + threadIdx.x;
   const int kz = blockIdx.y;
   if (kx >= lh) return;
-  const int64_t base = kx + (int64_t)d.lp * ny * kz;
+  const int64_t base = kx + d.srow(1, kz), st = d.ssj();
   double *PP = reinterpret_cast<double *>(d.ypiv) + base;
   double *HH = reinterpret_cast<double *>(d.ypiv) + (int64_t)d.lp * ny * d.nz + base;
   const double shift = d.ak1[kx] + d.ak3[kz];
@@ -1197,8 +1273,8 @@ __global__ void k_ypivots(TGDev d) {
     // (src/possion3d_fishpack_reform.f90:53-58): phi(ny) = 0
     pp = (pinn && j == ny) ? 0.0 : 1.0 / (b - h * d.amph[j]);
     h = j < ny ? d.apph[j] * pp : 0.0;
-    PP[(int64_t)d.lp * (j - 1)] = pp;
-    HH[(int64_t)d.lp * (j - 1)] = h;
+    PP[st * (j - 1)] = pp;
+    HH[st * (j - 1)] = h;
   }
 }
 
@@ -1215,7 +1291,7 @@ __global__ void __launch_bounds__(256) k_ysolve_line(TGDev d) {
   const int lh = d.lh, ny = d.ny;
   const int kx = blockIdx.x * blockDim.x + threadIdx.x, kz = blockIdx.y;
   if (kx >= lh) return;
-  const int64_t base = kx + (int64_t)d.lp * ny * kz, st = d.lp;
+  const int64_t base = kx + d.srow(1, kz), st = d.ssj();
   C *__restrict__ S = reinterpret_cast<C *>(d.spec) + base;
   const double *__restrict__ PP = reinterpret_cast<const double *>(d.ypiv) + base;
   const double *__restrict__ HH = reinterpret_cast<const double *>(d.ypiv) + (int64_t)d.lp * ny * d.nz + base;
@@ -1294,12 +1370,12 @@ __global__ void __launch_bounds__(128) k_ysolve_pair(TGDev q, TGDev s) {
   if (p >= q.lh) return;
   const int kc = kz ? nz - kz : 0;
   const bool self = kc == kz;
-  const int64_t st = q.lp, sp = s.lp;
-  double2 *__restrict__ Z1 = reinterpret_cast<double2 *>(q.spec) + p + st * ny * kz;
-  double2 *__restrict__ Z2 = reinterpret_cast<double2 *>(q.spec) + p + st * ny * kc;
+  const int64_t st = q.ssj(), sp = s.ssj();
+  double2 *__restrict__ Z1 = reinterpret_cast<double2 *>(q.spec) + p + q.srow(1, kz);
+  double2 *__restrict__ Z2 = reinterpret_cast<double2 *>(q.spec) + p + q.srow(1, kc);
   // pivots of modes 2p and 2p + 1 side by side (16-byte aligned: sp even)
-  const double *__restrict__ PP = reinterpret_cast<const double *>(s.ypiv) + 2 * p + sp * ny * kz;
-  const double *__restrict__ HH = PP + sp * ny * s.nz;
+  const double *__restrict__ PP = reinterpret_cast<const double *>(s.ypiv) + 2 * p + s.srow(1, kz);
+  const double *__restrict__ HH = PP + sp * ny;
   double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
   for (int j0 = 1; j0 <= ny; j0 += YP) {
     double2 z1[YP], z2[YP], pv[YP];
@@ -1366,7 +1442,7 @@ __global__ void __launch_bounds__(128) k_ysolve_pair(TGDev q, TGDev s) {
 }
 
 // Inverse real transform along x (src/possion3d_FFT99.f90:461-485): the
-// block's lb spectral rows (contiguous, pitch lp) arrive by one bulk copy;
+// block's lb spectral rows arrive by one bulk copy each;
 // pairs of rows are rebuilt as one complex Hermitian-extended line and
 // transformed; phi ghosts copied (BC_WALL_DPH, src/BC_WALL.f90:342-364).
 // accumulate != 0 adds the result to phi (refinement sweep).  The FFT
@@ -1397,11 +1473,10 @@ __global__ void __launch_bounds__(256, BIG ? 2 : 3) k_ifftx(TGDev d, FFTPlan pl,
   }
   if (tid < 16) rad[tid] = pl.rad[tid];
   __syncthreads();
-  if (tid == 0) {
-    const uint32_t bytes = (uint32_t)(nrow * lp * sizeof(C));
-    mbar_expect_tx(&bar, bytes);
-    bulk_g2s(SP, reinterpret_cast<const C *>(d.spec) + (int64_t)lp * ((jbeg - 1) + (int64_t)ny * k), bytes, &bar);
-  }
+  const uint32_t rowb = (uint32_t)(lp * sizeof(C));
+  if (tid == 0) mbar_expect_tx(&bar, rowb * nrow);
+  __syncthreads();
+  if (tid < nrow) bulk_g2s(SP + tid * lp, reinterpret_cast<const C *>(d.spec) + d.srow(jbeg + tid, k), rowb, &bar);
   if (!mbar_wait(&bar, 0, d.err)) {
     mbar_wait(&bar, 0, d.err);
     return;
@@ -1632,7 +1707,8 @@ template <typename T> struct Prec {
     const void *dyn[] = {(const void *)k_rhs_tma<T>,      (const void *)k_adix<T>,           (const void *)k_adiz<T>,
                          (const void *)k_fftx<T, false>,  (const void *)k_ifftx<T, false>,   (const void *)k_fftz<T, false>,
                          (const void *)k_fftx<T, true>,   (const void *)k_ifftx<T, true>,    (const void *)k_fftz<T, true>,
-                         (const void *)k_adiy_smem<T>};
+                         (const void *)k_adiy_smem<T>,    (const void *)k_fftz_reg<8, -1>,   (const void *)k_fftz_reg<8, 1>,
+                         (const void *)k_fftz_reg<16, -1>, (const void *)k_fftz_reg<16, 1>};
     const void *row[] = {CHAPSIM_ADIXZ_RATTR(T, 2), CHAPSIM_ADIXZ_RATTR(T, 4), CHAPSIM_ADIXZ_RATTR(T, 6),
                          CHAPSIM_ADIXZ_RATTR(T, 8), CHAPSIM_ADIXZ_RATTR(T, 12)};
     // rows of short lines with wide halos: 64 rows of 8 + 24 values, 98 KB
@@ -1664,18 +1740,41 @@ template <typename T> struct Prec {
     return CHAPSIM_OK;
   }
 
+  // The z transforms of the spectral descriptor s, sign -1 forward: register-
+  // blocked in FP64 where the plan's blocks hold two lines or more, else (and
+  // for FP32 spectra, whose roundings the refined solve magnifies) in shared
+  // memory.
+  static int fftz(chapsim_ctx *c, const TGDev &s, int sign) {
+    RegPlan p = c->rz;
+    p.tw = c->fz.tw64;
+    int llz = 3;
+    const int per = p.nst ? p.n / std::min(p.R[0], std::min(p.R[1], p.nst == 3 ? p.R[2] : p.R[1])) : 0;
+    while (llz > 0 && (per << llz) > 256) --llz;
+    if (sizeof(T) == 8 && p.nst && llz >= 1) {
+      const int lz = 1 << llz;
+      const dim3 grid((s.lh + lz - 1) / lz, s.ny);
+      const size_t sm = (size_t)lz * p.n * sizeof(double2);
+      auto k = p.rmax > 8 ? (sign < 0 ? k_fftz_reg<16, -1> : k_fftz_reg<16, 1>)
+                          : (sign < 0 ? k_fftz_reg<8, -1> : k_fftz_reg<8, 1>);
+      k<<<grid, per << llz, sm, c->stream>>>(s, p, llz);
+    } else {
+      const int lz = fftz_lz(s.nz);
+      const dim3 grid((s.lh + lz - 1) / lz, s.ny);
+      if (c->fft_big)
+        k_fftz<T, true><<<grid, 256, fftz_smem(s.nz, lz), c->stream>>>(s, c->fz, lz, sign);
+      else
+        k_fftz<T, false><<<grid, 256, fftz_smem(s.nz, lz), c->stream>>>(s, c->fz, lz, sign);
+    }
+    LAUNCHED();
+    return CHAPSIM_OK;
+  }
+
   static int spectral_solve(chapsim_ctx *c, int accumulate, bool mark) {
     TGDev &d = c->d;
-    const int lz = fftz_lz(d.nz), lb = ifftx_lb(c);
+    const int lb = ifftx_lb(c);
+    int rc;
     if (mark) phase_mark(c, CHAPSIM_PH_FFTZ);
-    {
-      dim3 grid((d.lh + lz - 1) / lz, d.ny);
-      if (c->fft_big)
-        k_fftz<T, true><<<grid, 256, fftz_smem(d.nz, lz), c->stream>>>(d, c->fz, lz, -1);
-      else
-        k_fftz<T, false><<<grid, 256, fftz_smem(d.nz, lz), c->stream>>>(d, c->fz, lz, -1);
-      LAUNCHED();
-    }
+    if ((rc = fftz(c, d, -1))) return rc;
     if (mark) phase_mark(c, CHAPSIM_PH_YSOLVE);
     {
       const int bx = c->ys_bx;
@@ -1684,14 +1783,7 @@ template <typename T> struct Prec {
       LAUNCHED();
     }
     if (mark) phase_mark(c, CHAPSIM_PH_IFFTZ);
-    {
-      dim3 grid((d.lh + lz - 1) / lz, d.ny);
-      if (c->fft_big)
-        k_fftz<T, true><<<grid, 256, fftz_smem(d.nz, lz), c->stream>>>(d, c->fz, lz, +1);
-      else
-        k_fftz<T, false><<<grid, 256, fftz_smem(d.nz, lz), c->stream>>>(d, c->fz, lz, +1);
-      LAUNCHED();
-    }
+    if ((rc = fftz(c, d, +1))) return rc;
     if (mark) phase_mark(c, CHAPSIM_PH_IFFTX);
     {
       dim3 grid((d.ny + lb - 1) / lb, d.nz);
@@ -1838,6 +1930,7 @@ int init_kernels(chapsim_ctx *c) {
     k_ypivots<<<grid, 128, 0, c->stream>>>(d);
     LAUNCHED();
   }
+  c->rz = reg_plan(c->d.nz);
   c->fft_big = false;
   for (int s2 = 0; s2 < 16; ++s2)
     if (c->fx.rad[s2] == 7 || c->fx.rad[s2] == 11 || c->fz.rad[s2] == 7 || c->fz.rad[s2] == 11) c->fft_big = true;
@@ -1880,7 +1973,7 @@ __global__ void __launch_bounds__(128) k_xnp_fwd(TGDev d, TGDev s, const double 
   const double *src = d.rhsphi + d.sy * j + d.sz * k;
   for (int i = threadIdx.x; i < nx; i += blockDim.x) xrow[i] = src[i];
   __syncthreads();
-  double2 *dst = reinterpret_cast<double2 *>(s.spec) + (int64_t)s.lp * (j - 1) + (int64_t)s.lp * s.ny * k;
+  double2 *dst = reinterpret_cast<double2 *>(s.spec) + s.srow(j, k);
   for (int m = threadIdx.x; m < s.lp; m += blockDim.x) {
     double acc = 0.0;
     if (m < nx)
@@ -1892,7 +1985,7 @@ __global__ void __launch_bounds__(128) k_xnp_fwd(TGDev d, TGDev s, const double 
 __global__ void __launch_bounds__(128) k_xnp_bwd(TGDev d, TGDev s, const double *__restrict__ bt) {
   extern __shared__ double xrow[];
   const int j = blockIdx.x + 1, k = blockIdx.y, nx = d.nx, ny = d.ny;
-  const double2 *src = reinterpret_cast<const double2 *>(s.spec) + (int64_t)s.lp * (j - 1) + (int64_t)s.lp * s.ny * k;
+  const double2 *src = reinterpret_cast<const double2 *>(s.spec) + s.srow(j, k);
   for (int i = threadIdx.x; i < nx; i += blockDim.x) xrow[i] = src[i].x;
   __syncthreads();
   double *dst = d.phi + d.sy * j + d.sz * k;
@@ -1981,7 +2074,7 @@ __global__ void __launch_bounds__(256) k_xnp_qfwd(TGDev d, TGDev s, FFTPlan pl, 
     const double2 z = res[swz((r >> 1) * nx + n)];
     double y = (r & 1) ? z.y : z.x;
     if (sinq && (m & 1)) y = -y;
-    S[m + 2 * (int64_t)s.lp * ((jbeg + r - 1) + (int64_t)ny * k)] = y * rscal;  // mode m: line m / 2, part m % 2
+    S[m + 2 * s.srow(jbeg + r, k)] = y * rscal;  // mode m: line m / 2, part m % 2
   }
 }
 
@@ -2007,9 +2100,9 @@ __global__ void __launch_bounds__(256) k_xnp_qbwd(TGDev d, TGDev s, FFTPlan pl, 
   const uint32_t rowb = (uint32_t)(nx * sizeof(double));
   if (tid == 0) mbar_expect_tx(&bar, rowb * (uint32_t)nrow);
   __syncthreads();
-  const double *S = reinterpret_cast<const double *>(s.spec) + 2 * (int64_t)s.lp * ((jbeg - 1) + (int64_t)ny * k);
+  const double *S = reinterpret_cast<const double *>(s.spec) + 2 * s.srow(jbeg, k);
   for (int r = tid; r < nrow; r += blockDim.x)
-    bulk_g2s(in + (size_t)r * nx, S + 2 * (int64_t)s.lp * r, rowb, &bar);
+    bulk_g2s(in + (size_t)r * nx, S + 2 * s.ssj() * r, rowb, &bar);
   for (int t = tid; t < (lb - nrow) * nx; t += blockDim.x) in[(size_t)nrow * nx + t] = 0.0;
   if (!mbar_wait(&bar, 0, d.err)) {
     mbar_wait(&bar, 0, d.err);  // let copies in flight land before the block exits
@@ -2094,14 +2187,9 @@ int xnp_pois3d(chapsim_ctx *c, bool mark) {
     k_xnp_fwd<<<rows, 128, sm, c->stream>>>(d, s, c->xnp_f);
   LAUNCHED();
   typedef Prec<double> P;
-  const int lz = P::fftz_lz(d.nz);
-  const dim3 gz((z.lh + lz - 1) / lz, d.ny);
+  int rc;
   if (mark) phase_mark(c, CHAPSIM_PH_FFTZ);
-  if (c->fft_big)
-    k_fftz<double, true><<<gz, 256, P::fftz_smem(d.nz, lz), c->stream>>>(z, c->fz, lz, -1);
-  else
-    k_fftz<double, false><<<gz, 256, P::fftz_smem(d.nz, lz), c->stream>>>(z, c->fz, lz, -1);
-  LAUNCHED();
+  if ((rc = P::fftz(c, z, -1))) return rc;
   if (mark) phase_mark(c, CHAPSIM_PH_YSOLVE);
   if (q) {
     dim3 grid((qs.lh + 127) / 128, d.nz / 2 + 1);
@@ -2113,11 +2201,7 @@ int xnp_pois3d(chapsim_ctx *c, bool mark) {
   }
   LAUNCHED();
   if (mark) phase_mark(c, CHAPSIM_PH_IFFTZ);
-  if (c->fft_big)
-    k_fftz<double, true><<<gz, 256, P::fftz_smem(d.nz, lz), c->stream>>>(z, c->fz, lz, +1);
-  else
-    k_fftz<double, false><<<gz, 256, P::fftz_smem(d.nz, lz), c->stream>>>(z, c->fz, lz, +1);
-  LAUNCHED();
+  if ((rc = P::fftz(c, z, +1))) return rc;
   if (mark) phase_mark(c, CHAPSIM_PH_IFFTX);
   if (q && c->fft_big)
     k_xnp_qbwd<true><<<qgrid, 256, smq, c->stream>>>(d, qs, c->fx, c->xnp_qw, lb, sinq);

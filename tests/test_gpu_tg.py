@@ -318,3 +318,15 @@ def test_adi_factor_wider_bands(dt, ren):
         g.solverrk3_mom_tg(ns)
         o.substep(ns)
         compare(g, o, tag=f"ns{ns}")
+
+
+@pytest.mark.parametrize("nz", [8, 10, 14, 22, 24, 30, 36, 50, 54, 66, 98, 110, 126, 144, 150, 210, 242, 256, 264, 352, 450, 512])
+def test_z_transform_lengths(nz):
+    """The register-blocked z transforms over their radices (2 to 16, composite
+    and prime), two and three stages, and lines per block; 242 = 2 x 11 x 11
+    takes three stages."""
+    g, o = pair(10, 5, nz, seed=4)
+    g.solverrk3_mom_tg(0)
+    o.substep(0)
+    compare(g, o, tag=f"nz {nz}")
+
