@@ -153,7 +153,7 @@ struct chapsim_ctx {
 
   chapsim::TGDev d{};
   chapsim::FFTPlan fx{}, fz{};
-  chapsim::RegPlan rz{};  // the z transform's register-blocked stages (none: nst = 0)
+  chapsim::RegPlan rx{}, rz{};  // the transforms' register-blocked stages (none: nst = 0)
   // host mesh copies
   std::vector<double> ynd, ycc, dyfi, dyci, wff, wfb;
   double area_inlet = 0.0;

@@ -227,15 +227,16 @@ template <int SG> struct Dft<14, SG> : DftSplit<2, 7, SG> {};
 template <int SG> struct Dft<15, SG> : DftSplit<3, 5, SG> {};
 template <int SG> struct Dft<16, SG> : DftSplit<4, 4, SG> {};
 
-// The plan of n points: two radices up to 16, else three, chosen for the
-// smallest largest one (registers), then the smallest sum.
-inline RegPlan reg_plan(int n) {
+// The plan of n points: two radices up to `most`, else three (up to 16 where
+// `most` does not suffice), chosen for the smallest largest one (registers),
+// then the smallest sum.
+inline RegPlan reg_plan(int n, int most = 16) {
   static const int rad[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 14, 15, 16};
   RegPlan p{n, 0, 0, {1, 1, 1}, nullptr};
   int best = 1 << 30;
   auto take = [&](int a, int b, int c) {
     const int m = a > b ? (a > c ? a : c) : (b > c ? b : c), cost = 64 * m + a + b + c;
-    if (cost >= best) return;
+    if (m > most || cost >= best) return;
     best = cost;
     p.nst = c > 1 ? 3 : 2;
     p.rmax = m;
@@ -251,7 +252,16 @@ inline RegPlan reg_plan(int n) {
     for (int b : rad)
       for (int c : rad)
         if (a * b * c == n) take(a, b, c);
+  if (!p.nst && most < 16) return reg_plan(n);
   return p;
+}
+
+// Butterflies of the stage that has most: threads per line
+inline int reg_per(const RegPlan &p) {
+  if (!p.nst) return 0;
+  int m = p.R[0] < p.R[1] ? p.R[0] : p.R[1];
+  if (p.nst == 3 && p.R[2] < m) m = p.R[2];
+  return p.n / m;
 }
 
 // f(integral constant R) for the plan's radix r, R <= RMAX
@@ -283,6 +293,72 @@ template <int R, int SG> __device__ __forceinline__ void reg_twiddle(double2 (&v
     if (SG > 0) t.y = -t.y;
     v[r] = cmul(v[r], t);
   }
+}
+
+// Position of element p of a line-major buffer: the low three bits XORed with
+// the two groups of three above them, a permutation inside every aligned
+// group of eight. The first stage writes at stride R (8 or 16 elements of 16
+// bytes); permuted, those writes and the contiguous reads spread over all
+// banks.
+__device__ __forceinline__ int swz2(int p) { return p ^ ((p >> 3) & 7) ^ ((p >> 6) & 7); }
+
+// One line of pl.n points at `base` of the buffer A, butterfly j of every
+// stage by the calling thread: load(i) gives point i, store(k, value) takes
+// result k.  Every thread of the block calls it (act: the line exists).  KEEP
+// puts a barrier before the stores, for a store that writes A.
+template <int RMAX, int SG, bool KEEP, typename L, typename S>
+__device__ __forceinline__ void reg_line(const RegPlan &pl, double2 *A, int base, int j, bool act, L load, S store) {
+  const int n = pl.n;
+  with_radix<RMAX>(pl.R[0], [&](auto tag) {
+    constexpr int R = decltype(tag)::value;
+    const int nb = n / R;
+    if (act && j < nb) {
+      double2 v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = load(j + r * nb);
+      Dft<R, SG>::run(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) A[swz2(base + j * R + r)] = v[r];
+    }
+  });
+  __syncthreads();
+  int Ns = pl.R[0];
+  if (pl.nst == 3) {
+    with_radix<RMAX>(pl.R[1], [&](auto tag) {
+      constexpr int R = decltype(tag)::value;
+      const int nb = n / R, jq = j / Ns, k = j - jq * Ns;
+      double2 v[R];
+      if (act && j < nb) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = A[swz2(base + j + r * nb)];
+        reg_twiddle<R, SG>(v, pl.tw, k * (n / (Ns * R)));
+        Dft<R, SG>::run(v);
+      }
+      __syncthreads();
+      if (act && j < nb) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) A[swz2(base + jq * Ns * R + k + r * Ns)] = v[r];
+      }
+    });
+    __syncthreads();
+    Ns *= pl.R[1];
+  }
+  with_radix<RMAX>(pl.nst == 3 ? pl.R[2] : pl.R[1], [&](auto tag) {
+    constexpr int R = decltype(tag)::value;
+    const int nb = n / R;  // = Ns
+    double2 v[R];
+    if (act && j < nb) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = A[swz2(base + j + r * nb)];
+      reg_twiddle<R, SG>(v, pl.tw, j);
+      Dft<R, SG>::run(v);
+    }
+    if (KEEP) __syncthreads();
+    if (act && j < nb) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) store(j + r * nb, v[r]);
+    }
+  });
 }
 
 }  // namespace chapsim

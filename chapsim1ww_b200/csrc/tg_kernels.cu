@@ -1104,6 +1104,50 @@ __global__ void __launch_bounds__(256, BIG ? 2 : 3) k_fftx(TGDev d, SubParams sp
   }
 }
 
+// The FP64 form of k_fftx with register-blocked lines (fft_reg.cuh): the
+// points of the first stage are the divergences, formed from global memory
+// (each value of u, v, w serves up to three of them out of the L1 cache); a
+// last crossing of shared memory separates the two rows of a line.  `per`
+// threads per line.
+template <int RMAX>
+__global__ void __launch_bounds__(256, RMAX > 8 ? 2 : 3) k_fftx_reg(TGDev d, SubParams sp, RegPlan pl, int per, int mode) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  double2 *A = reinterpret_cast<double2 *>(smem_raw);
+  const int nx = d.nx, ny = d.ny, lh = d.lh, k = blockIdx.y;
+  const int nl = blockDim.x / per, p = threadIdx.x / per, j = threadIdx.x - p * per;
+  const int j0 = 1 + 2 * (blockIdx.x * nl + p);  // the line's rows j0, j0 + 1
+  const bool act = j0 <= ny, two = j0 < ny;
+  const int64_t sy = d.sy, c0 = sy * j0 + d.sz * k, ozp = k + 1 == d.nz ? -d.sz * (d.nz - 1) : d.sz;
+  const double coe0 = 1.0 / (d.dt * sp.alp);
+  const double *__restrict__ U = d.u, *__restrict__ V = d.v, *__restrict__ W = d.w, *__restrict__ DR = d.drho;
+  auto div = [&](int64_t c, int64_t oxp, double dyfi) {
+    double dv = (U[c + oxp] - U[c]) * d.dxi + (V[c + sy] - V[c]) * dyfi + (W[c + ozp] - W[c]) * d.dzi;
+    if (DR) dv += DR[c];  // DIVG_io: + DrhoDtP
+    const double val = dv * coe0;
+    if (!d.skip_rhs) d.rhsphi[c] = val;
+    return val;
+  };
+  const double f0 = act ? d.dyfi[j0] : 0.0, f1 = two ? d.dyfi[j0 + 1] : 0.0;
+  auto load = [&](int i) {
+    const int64_t c = c0 + i;
+    if (mode == 1) return make_double2(d.rhsphi[c], two ? d.rhsphi[c + sy] : 0.0);
+    const int64_t oxp = i + 1 == nx ? 1 - nx : 1;
+    return make_double2(div(c, oxp, f0), two ? div(c + sy, oxp, f1) : 0.0);
+  };
+  reg_line<RMAX, -1, true>(pl, A, p * nx, j, act, load, [&](int kk, double2 v) { A[swz2(p * nx + kk)] = v; });
+  __syncthreads();
+  const double scale = 0.5 / nx;
+  double2 *S = reinterpret_cast<double2 *>(d.spec);
+  for (int t = threadIdx.x; t < nl * lh; t += blockDim.x) {
+    const int q = t / lh, kx = t - q * lh, jq = 1 + 2 * (blockIdx.x * nl + q);
+    if (jq > ny) break;
+    const double2 z = A[swz2(q * nx + kx)], zc = A[swz2(q * nx + (kx == 0 ? 0 : nx - kx))];
+    S[kx + d.srow(jq, k)] = make_double2((z.x + zc.x) * scale, (z.y - zc.y) * scale);
+    // -i (z - conj zc) / 2
+    if (jq < ny) S[kx + d.srow(jq + 1, k)] = make_double2((z.y + zc.y) * scale, (zc.x - z.x) * scale);
+  }
+}
+
 // Complex transform along z for lz consecutive kx at row j
 // (src/possion3d_FFT99.f90:301-317 forward with 1/nz and the (1,1,1) mode
 // zeroed (:324-327); :448-458 inverse).  The block's nz rows of lz spectral
@@ -1512,6 +1556,44 @@ __global__ void __launch_bounds__(256, BIG ? 2 : 3) k_ifftx(TGDev d, FFTPlan pl,
   }
 }
 
+// The FP64 form of k_ifftx with register-blocked lines: the first stage takes
+// its points from the spectral rows in global memory (X and its mirror image
+// for the upper half), the last writes phi: no staging, no separate packing
+// and unpacking.  Radices up to 8 (80 registers, three blocks of 256 threads
+// per SM) beat two of 16 here: 256x192x256 84 -> 72 us (76 with 16 x 16),
+// 384x192x192 119 -> 89, 210x99x154 54 -> 26.
+template <int RMAX>
+__global__ void __launch_bounds__(256, RMAX > 8 ? 2 : 3) k_ifftx_reg(TGDev d, RegPlan pl, int per) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  double2 *A = reinterpret_cast<double2 *>(smem_raw);
+  const int nx = d.nx, ny = d.ny, k = blockIdx.y;
+  const int nl = blockDim.x / per, p = threadIdx.x / per, j = threadIdx.x - p * per;
+  const int j0 = 1 + 2 * (blockIdx.x * nl + p);
+  const bool act = j0 <= ny, two = j0 < ny;
+  const double2 *__restrict__ S0 = reinterpret_cast<const double2 *>(d.spec) + d.srow(act ? j0 : 1, k);
+  const double2 *__restrict__ S1 = S0 + (two ? d.ssj() : 0);
+  double *phi = d.phi + d.sy * j0 + d.sz * k;
+  auto load = [&](int i) {
+    const bool up = 2 * i > nx;
+    const int kx = up ? nx - i : i;
+    double2 x0 = S0[kx], x1 = S1[kx];
+    if (!two) x1 = make_double2(0.0, 0.0);
+    if (i == 0 || 2 * i == nx) x0.y = x1.y = 0.0;
+    // Z(k) = X0 + i X1; Z(n - k) = conj(X0) + i conj(X1)
+    return up ? make_double2(x0.x + x1.y, x1.x - x0.y) : make_double2(x0.x - x1.y, x0.y + x1.x);
+  };
+  auto store = [&](int i, double2 v) {
+    phi[i] = v.x;
+    if (j0 == 1) phi[i - d.sy] = v.x;  // BC_WALL_DPH: ghost rows by copy
+    if (j0 == ny) phi[i + d.sy] = v.x;
+    if (two) {
+      phi[i + d.sy] = v.y;
+      if (j0 + 1 == ny) phi[i + 2 * d.sy] = v.y;
+    }
+  };
+  reg_line<RMAX, 1, false>(pl, A, p * nx, j, act, load, store);
+}
+
 // FP64 residual of the discrete Poisson operator the spectral solver inverts
 // (the operator of CHECK_FFT_SOLVER, src/PRESSURE_CORRECTION.f90:159-202):
 // res = RHSLLPHI - [d_xx + d_zz + L_y] phi, with L_y the folded Neumann
@@ -1708,7 +1790,8 @@ template <typename T> struct Prec {
                          (const void *)k_fftx<T, false>,  (const void *)k_ifftx<T, false>,   (const void *)k_fftz<T, false>,
                          (const void *)k_fftx<T, true>,   (const void *)k_ifftx<T, true>,    (const void *)k_fftz<T, true>,
                          (const void *)k_adiy_smem<T>,    (const void *)k_fftz_reg<8, -1>,   (const void *)k_fftz_reg<8, 1>,
-                         (const void *)k_fftz_reg<16, -1>, (const void *)k_fftz_reg<16, 1>};
+                         (const void *)k_fftz_reg<16, -1>, (const void *)k_fftz_reg<16, 1>, (const void *)k_fftx_reg<8>,
+                         (const void *)k_fftx_reg<16>,     (const void *)k_ifftx_reg<8>,     (const void *)k_ifftx_reg<16>};
     const void *row[] = {CHAPSIM_ADIXZ_RATTR(T, 2), CHAPSIM_ADIXZ_RATTR(T, 4), CHAPSIM_ADIXZ_RATTR(T, 6),
                          CHAPSIM_ADIXZ_RATTR(T, 8), CHAPSIM_ADIXZ_RATTR(T, 12)};
     // rows of short lines with wide halos: 64 rows of 8 + 24 values, 98 KB
@@ -1727,9 +1810,46 @@ template <typename T> struct Prec {
     return CHAPSIM_OK;
   }
 
+  // Launch shape of the register-blocked x transforms: false where the plan
+  // has none or its lines take more than 256 threads.  About 128 threads a
+  // block at radices above 8 (128 registers each), 256 otherwise.
+  struct XReg {
+    RegPlan p;
+    int per, threads;
+    dim3 grid;
+    size_t smem;
+  };
+  static bool x_reg(const chapsim_ctx *c, XReg &x) {
+    x.p = c->rx;
+    x.p.tw = c->fx.tw64;
+    if (!x.p.nst) return false;
+    x.per = reg_per(x.p);
+    if (x.per > 256) return false;
+    const int pairs = (c->d.ny + 1) / 2;
+    int nl = std::max(1, (x.p.rmax > 8 ? 128 : 256) / x.per);
+    nl = std::min(nl, pairs);
+    x.threads = nl * x.per;
+    x.grid = dim3((pairs + nl - 1) / nl, c->d.nz);
+    x.smem = (((size_t)nl * x.p.n + 7) & ~(size_t)7) * sizeof(double2);
+    return true;
+  }
+
   // mode 0: divergence of q; 1: stored RHSLLPHI; 2: residual buffer
   static int fftx(chapsim_ctx *c, int ns, int mode) {
     TGDev &d = c->d;
+    XReg x;
+    // Powers of two keep the staged kernel: its index arithmetic is shifts and
+    // its inputs arrive by bulk copies (256 points: 150 us at 256x192x256
+    // against 171; 1024: 1415 against 1452 at 1024x384x256), where other
+    // lengths spend their time on divisions (384: 247 against 203 us at
+    // 384x192x192; 210: 80 against 62 us at 210x99x154).
+    const bool pow2 = (d.nx & (d.nx - 1)) == 0;
+    if (sizeof(T) == 8 && mode != 2 && !pow2 && x_reg(c, x)) {
+      auto k = x.p.rmax > 8 ? k_fftx_reg<16> : k_fftx_reg<8>;
+      k<<<x.grid, x.threads, x.smem, c->stream>>>(d, c->sp[ns], x.p, x.per, mode);
+      LAUNCHED();
+      return CHAPSIM_OK;
+    }
     const int lb = fftx_lb(c);
     dim3 grid((d.ny + lb - 1) / lb, d.nz);
     if (c->fft_big)
@@ -1748,7 +1868,7 @@ template <typename T> struct Prec {
     RegPlan p = c->rz;
     p.tw = c->fz.tw64;
     int llz = 3;
-    const int per = p.nst ? p.n / std::min(p.R[0], std::min(p.R[1], p.nst == 3 ? p.R[2] : p.R[1])) : 0;
+    const int per = reg_per(p);
     while (llz > 0 && (per << llz) > 256) --llz;
     if (sizeof(T) == 8 && p.nst && llz >= 1) {
       const int lz = 1 << llz;
@@ -1785,7 +1905,12 @@ template <typename T> struct Prec {
     if (mark) phase_mark(c, CHAPSIM_PH_IFFTZ);
     if ((rc = fftz(c, d, +1))) return rc;
     if (mark) phase_mark(c, CHAPSIM_PH_IFFTX);
-    {
+    XReg x;
+    if (sizeof(T) == 8 && !accumulate && x_reg(c, x)) {
+      auto k = x.p.rmax > 8 ? k_ifftx_reg<16> : k_ifftx_reg<8>;
+      k<<<x.grid, x.threads, x.smem, c->stream>>>(d, x.p, x.per);
+      LAUNCHED();
+    } else {
       dim3 grid((d.ny + lb - 1) / lb, d.nz);
       if (c->fft_big)
         k_ifftx<T, true><<<grid, 256, ifftx_smem(d.nx, d.lp, lb), c->stream>>>(d, c->fx, lb, accumulate);
@@ -1930,6 +2055,7 @@ int init_kernels(chapsim_ctx *c) {
     k_ypivots<<<grid, 128, 0, c->stream>>>(d);
     LAUNCHED();
   }
+  c->rx = reg_plan(c->d.nx, 8);
   c->rz = reg_plan(c->d.nz);
   c->fft_big = false;
   for (int s2 = 0; s2 < 16; ++s2)

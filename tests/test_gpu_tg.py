@@ -330,3 +330,12 @@ def test_z_transform_lengths(nz):
     o.substep(0)
     compare(g, o, tag=f"nz {nz}")
 
+
+@pytest.mark.parametrize("nx", [8, 10, 14, 22, 24, 36, 50, 54, 66, 98, 126, 144, 150, 210, 242, 256, 264, 352, 450, 512])
+def test_x_transform_lengths(nx):
+    """The register-blocked x transforms over their radices and stages, with
+    an odd row count (the last line holds one row)."""
+    g, o = pair(nx, 5, 8, seed=4)
+    g.solverrk3_mom_tg(0)
+    o.substep(0)
+    compare(g, o, tag=f"nx {nx}")
