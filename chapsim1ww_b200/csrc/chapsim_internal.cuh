@@ -226,6 +226,8 @@ struct chapsim_ctx {
   cudaGraphExec_t io_graph[2] = {nullptr, nullptr};  // one step starting from io_cur = 0 / 1
   // TMA descriptors of the IO momentum RHS: u, v, w, p, mu0 + mu, g[0][0..2], g[1][0..2], EXPLT0
   CUtensorMap io_maps[14];
+  CUtensorMap si_maps[4];  // semi-implicit scheme: mu, DRHOI_STG 1-3
+  bool use_tma_si = false;
   bool use_tma_io = false;
   int io_nzc = 16;  // z planes per block of the TMA momentum RHS
   bool si_smem_set = false;  // semi-implicit solve kernels got their shared-memory limit
@@ -300,6 +302,7 @@ int io_mom(chapsim_ctx *c, int ns, bool prep);
 // then the x, z, y factor solves writing G* into the other G buffer
 int io_mom_si(chapsim_ctx *c, int ns, int *npart);
 int io_factor_si(chapsim_ctx *c, int ns);
+int io_si_setup(chapsim_ctx *c);
 int io_reduce(chapsim_ctx *c, int what, double *host_out);
 int io_correction(chapsim_ctx *c, int ns);
 int io_init_maps(chapsim_ctx *c);

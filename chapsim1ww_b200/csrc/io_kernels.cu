@@ -1455,6 +1455,18 @@ int io_init_maps(chapsim_ctx *c) {
       return CHAPSIM_ERR_CUDA;
     }
   }
+  if (io.visc) {
+    void *fs[4] = {io.mu, io.drhoi[0], io.drhoi[1], io.drhoi[2]};
+    for (int m = 0; m < 4; ++m)
+      if (encode(&c->si_maps[m], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, fs[m], dims, strides, box, es,
+                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+        c->err = "cuTensorMapEncodeTiled failed";
+        return CHAPSIM_ERR_CUDA;
+      }
+    const int rc = io_si_setup(c);
+    if (rc) return rc;
+  }
   int dev = 0, optin = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));

@@ -90,3 +90,25 @@ def test_io_implicit_density_correction_active():
     g.solverrk3_mom_io(1)
     o.mom(1)
     compare(g, o, FLOW + ("ex0x", "ex0y", "ex0z"), tag="planted density")
+
+
+# nx >= 36 and ny >= 8 run the z-marching right-hand side (36: one partial
+# second x tile, 66 x 9: partial tiles in x and y; nz 9 planes a march); the
+# line solves take lengths with 1, 2 and 32 chunks
+@pytest.mark.parametrize("gravdir", [0, 1, 2])
+@pytest.mark.parametrize("dims", [(36, 8, 10), (66, 9, 18), (40, 33, 64), (132, 10, 8)])
+def test_io_implicit_marching_edges(dims, gravdir):
+    """Variable properties from an uneven enthalpy field, buoyancy along x or
+    y, against the oracle after each of the first two substeps (velocities,
+    mass fluxes, explicit terms, thermal fields)."""
+    g, o = pair(*dims, thermal=1, gravdir=gravdir, f_a=0.3 if gravdir else 0.0)
+    rng = np.random.default_rng(11)
+    rhoh = o.get("rho") * (0.3 * rng.standard_normal(g.shape)).clip(-0.8, 0.8)
+    o.set("rhoh", rhoh)
+    g.set_field("rhoh", rhoh)
+    for ns in (1, 2):
+        g.solverrk3_eng_io(ns)
+        o.eng(ns)
+        g.solverrk3_mom_io(ns)
+        o.mom(ns)
+        compare(g, o, ("u", "v", "w", "gx", "gy", "gz", "ex0x", "ex0y", "ex0z") + THERMAL, tag=f"ns{ns}")
