@@ -1409,7 +1409,10 @@ int chapsim_set_props_mode(chapsim_ctx *ctx, int mode, const chapsim_props *pe) 
     CKC(cudaMemcpyAsync(b, src.par, npar_b, cudaMemcpyDeviceToDevice, ctx->stream));
     CKC(cudaMemcpyAsync(b + npar, src.wt, nwt_b, cudaMemcpyDeviceToDevice, ctx->stream));
     CKC(cudaMemcpyAsync(b + npar + nwt, src.gate, chapsim_mlp::kMaxGateBins, cudaMemcpyDeviceToDevice, ctx->stream));
+    std::vector<float> par(chapsim_mlp::NP);
+    CKC(cudaMemcpyAsync(par.data(), src.par, npar_b, cudaMemcpyDeviceToHost, ctx->stream));
     CKC(cudaStreamSynchronize(ctx->stream));
+    chapsim_mlp::set_weights(ctx->mlp_w, par.data());
     ctx->mlp = src;
     ctx->mlp.par = reinterpret_cast<const float *>(b);
     ctx->mlp.wt = reinterpret_cast<const uint16_t *>(b + npar);

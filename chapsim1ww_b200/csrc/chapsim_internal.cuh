@@ -235,6 +235,7 @@ struct chapsim_ctx {
   // model (a copy of a trained engine's model in context-owned buffers)
   int props_mode = CHAPSIM_PROPS_TABLE;
   chapsim_mlp::MlpDev mlp{};
+  chapsim_mlp::MlpW mlp_w{};
   void *mlp_buf = nullptr;
   bool mlp_smem_set = false;
   // on-device statistics (partials, xz averages, time averages) and the

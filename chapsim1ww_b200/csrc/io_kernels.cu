@@ -334,21 +334,33 @@ __global__ void __launch_bounds__(IO_BX *IO_BY) k_io_props_only(TGDev d, IODev i
 // substep (|dx| ~ 1e-4); a tile in which any model cell moves further than
 // kTaylorMax evaluates the model a second time at h2.  This halves the tanh
 // evaluations; the elementwise work between the layers runs on packed FP32
-// pairs, and the kernel is bound by its instruction issue rate.
-__global__ void __launch_bounds__(chapsim_mlp::TILE, 3) k_io_eng_props_mlp(TGDev d, IODev io, chapsim_mlp::MlpDev M) {
+// pairs.  One CTA per SM, four groups of four warps that each walk tiles of
+// their own: 9.07 -> 8.72 ms at 1024 x 384 x 256 (the round trip through the
+// tensor pipe is hidden by 16 warps instead of 12).  The FP32 weights come as
+// the kernel's parameter: as shared-memory broadcasts they took 39 % of the
+// shared-memory data pipe next to the MMA's operand reads (25 %), 8.72 ->
+// 7.93 ms.  Now the warps issue 52 % of the cycles, the special-function pipe
+// is busy 42 %, FMA 40 %, tensor 19 %; what is left are the waits for the
+// layer-2 MMA and tensor memory (no room for more tiles in flight).
+__global__ void __launch_bounds__(chapsim_mlp::TILE *chapsim_mlp::SmemD::G, 1)
+    k_io_eng_props_mlp(TGDev d, IODev io, chapsim_mlp::MlpDev M, const __grid_constant__ chapsim_mlp::MlpW W) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   chapsim_mlp::SmemD &s = chapsim_mlp::smem_of<chapsim_mlp::SmemD>(smem_raw);
-  chapsim_mlp::cta_setup_d(s, M);
+  chapsim_mlp::cta_setup(s, M);
+  const chapsim_mlp::Grp grp = chapsim_mlp::grp_of(s);
   uint32_t phase = 0;
   const int64_t n = d.sz * d.nz;
   const int64_t ntiles = (n + chapsim_mlp::TILE - 1) / chapsim_mlp::TILE;
   const int64_t rows = d.ny + 2;
   const double hinv = 1.0 / M.hhalf;
-  // The thread's cell advances by a fixed stride per tile: its x index and
-  // row j follow incrementally instead of by two 64-bit divisions per cell.
-  const int64_t stride = (int64_t)gridDim.x * chapsim_mlp::TILE;
+  // Group g of block b starts at tile b + g gridDim.x (few tiles spread over
+  // all blocks first).  The thread's cell advances by a fixed stride per tile:
+  // its x index and row j follow incrementally instead of by two 64-bit
+  // divisions per cell.
+  const int64_t tstep = (int64_t)gridDim.x * chapsim_mlp::SmemD::G, tile0 = blockIdx.x + (int64_t)gridDim.x * grp.g;
+  const int64_t stride = tstep * chapsim_mlp::TILE;
   const int sx = (int)(stride % d.nx), sj = (int)((stride / d.nx) % rows);
-  int64_t c = (int64_t)blockIdx.x * chapsim_mlp::TILE + threadIdx.x;
+  int64_t c = tile0 * chapsim_mlp::TILE + grp.r;
   int ix = (int)(c % d.nx), j = (int)((c / d.nx) % rows);
   // the next tile's inputs are loaded while the current one is evaluated
   double nD = 1.0, nmu = 0.0, nrh = 0.0;
@@ -357,7 +369,7 @@ __global__ void __launch_bounds__(chapsim_mlp::TILE, 3) k_io_eng_props_mlp(TGDev
     nmu = io.mu[c];
     nrh = io.rhoh[c];
   }
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, c += stride) {
+  for (int64_t tile = tile0; tile < ntiles; tile += tstep, c += stride) {
     const bool valid = c < n;
     const bool interior = valid && j >= 1 && j <= d.ny;
     const double dold = nD, muold = nmu, rh = interior ? nrh : 0.0;
@@ -380,7 +392,7 @@ __global__ void __launch_bounds__(chapsim_mlp::TILE, 3) k_io_eng_props_mlp(TGDev
     const double h1 = rh / dold;
     const double x1 = (h1 - M.hmid) * hinv;
     float y[chapsim_mlp::NO], dy[chapsim_mlp::NO];
-    chapsim_mlp::tile_eval_d(s, (float)x1, y, dy, phase, d.err);  // a failed wait: s.fail, read below
+    chapsim_mlp::tile_eval_d(s, W, grp, (float)x1, y, dy, phase, d.err);  // a failed wait: s.fail, read below
     int bad = 0;
     double D = dold;
     if (interior) {
@@ -403,12 +415,12 @@ __global__ void __launch_bounds__(chapsim_mlp::TILE, 3) k_io_eng_props_mlp(TGDev
     const bool keep = io.shortcuts && fabs(h2) < 1.0e-10;
     const bool model2 = interior && !keep && chapsim_spl::inside_h(io.tab, h2) &&
                         chapsim_mlp::gate_step(s, M, h2);
-    const bool again = __syncthreads_or(model2 && fabs(x2 - x1) > chapsim_mlp::kTaylorMax);
-    if (s.fail) break;  // block-uniform after the barrier
+    const bool again = chapsim_mlp::grp_or(s, grp, model2 && fabs(x2 - x1) > chapsim_mlp::kTaylorMax);
+    if (s.fail[grp.g]) break;  // group-uniform after the barrier
     float y2[chapsim_mlp::NO];
-    if (again && threadIdx.x == 0) atomicAdd(io.model_again, 1ull);
+    if (again && grp.r == 0) atomicAdd(io.model_again, 1ull);
     if (again) {
-      if (!chapsim_mlp::tile_eval(s, (float)x2, y2, phase, d.err)) break;
+      if (!chapsim_mlp::tile_eval(s, grp, (float)x2, y2, phase, d.err)) break;
     } else {
 #pragma unroll
       for (int q = 0; q < chapsim_mlp::NO; ++q) y2[q] = y[q] + dy[q] * (float)(x2 - x1);
@@ -452,11 +464,13 @@ __global__ void __launch_bounds__(chapsim_mlp::TILE, 3) k_io_eng_props_mlp(TGDev
 __global__ void __launch_bounds__(chapsim_mlp::TILE, 4) k_io_therm_props(TGDev d, IODev io, chapsim_mlp::MlpDev M,
                                                                          int use_mlp) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  chapsim_mlp::Smem *sp = nullptr;
+  chapsim_mlp::Smem1 *sp = nullptr;
+  chapsim_mlp::Grp grp{};
   uint32_t phase = 0;
   if (use_mlp) {
-    sp = &chapsim_mlp::smem_of(smem_raw);
+    sp = &chapsim_mlp::smem_of<chapsim_mlp::Smem1>(smem_raw);
     chapsim_mlp::cta_setup(*sp, M);
+    grp = chapsim_mlp::grp_of(*sp);
   }
   const int64_t n = d.sz * d.nz;
   const int64_t ntiles = (n + chapsim_mlp::TILE - 1) / chapsim_mlp::TILE;
@@ -469,7 +483,7 @@ __global__ void __launch_bounds__(chapsim_mlp::TILE, 4) k_io_therm_props(TGDev d
     const double h = interior ? io.h[c] : 0.0;
     const double x = use_mlp ? (h - M.hmid) / M.hhalf : 0.0;
     float y[chapsim_mlp::NO];
-    if (use_mlp && !chapsim_mlp::tile_eval(*sp, (float)x, y, phase, d.err)) break;
+    if (use_mlp && !chapsim_mlp::tile_eval(*sp, grp, (float)x, y, phase, d.err)) break;
     if (!interior || (io.shortcuts && fabs(h) < 1.0e-10)) continue;
     double T, D, Mu, K;
     bool ok = chapsim_spl::inside_h(io.tab, h);
@@ -1279,9 +1293,9 @@ int io_thermal_bc(chapsim_ctx *c) {
 }
 
 // The learned-property kernels take more than 48 KB of dynamic shared memory
-// (set once per context) and run persistently, three (energy substep, with
-// the derivative tile) or four CTAs of 128 threads per SM; each CTA holds 128
-// of the SM's 512 tensor-memory columns.
+// (set once per context) and run persistently, one CTA of four groups (energy
+// substep, with the derivative tile) or four CTAs of one group per SM; each
+// group of 128 threads holds 128 of the SM's 512 tensor-memory columns.
 int mlp_kernel_setup(chapsim_ctx *c) {
   if (c->mlp_smem_set) return CHAPSIM_OK;
   const void *fns[] = {(const void *)k_io_eng_props_mlp, (const void *)k_io_therm_props};
@@ -1320,7 +1334,7 @@ int io_eng(chapsim_ctx *c, int ns) {
   if (c->props_mode == CHAPSIM_PROPS_MLP) {
     int rc = mlp_kernel_setup(c);
     if (rc) return rc;
-    k_io_eng_props_mlp<<<mlp_grid(c, 3), chapsim_mlp::TILE, chapsim_mlp::kSmemDBytes, c->stream>>>(d, c->io, c->mlp);
+    k_io_eng_props_mlp<<<mlp_grid(c, 1), chapsim_mlp::TILE * chapsim_mlp::SmemD::G, chapsim_mlp::kSmemDBytes, c->stream>>>(d, c->io, c->mlp, c->mlp_w);
   } else {
     k_io_eng_props<<<g2, dim3(IO_BX, IO_BY), 0, c->stream>>>(d, c->io);
   }

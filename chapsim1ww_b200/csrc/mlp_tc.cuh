@@ -9,8 +9,9 @@
 // table by cubic splines, src/THERM_PROP_UPDATE.f90:129-205,
 // src/Flow_State.f90:1015-1070,1420-1581); the splines stay as the fallback.
 //
-// One CTA of 128 threads evaluates tiles of 128 cells (one cell per thread,
-// the MMA's M = 128 rows):
+// A group of 128 threads evaluates tiles of 128 cells (one cell per thread,
+// the MMA's M = 128 rows); a CTA holds one group, or four that share the
+// weights (the energy substep):
 //  - layer 1 on the CUDA cores in FP32 (tanh.approx.f32), the affine parts
 //    and every other elementwise step on packed FP32 pairs (.f32x2);
 //  - each activation vector is split into BF16 hi + lo parts (lo = the
@@ -22,7 +23,7 @@
 //    are issued by one thread as tcgen05.mma kind::f16 from shared-memory
 //    operands in the canonical no-swizzle K-major layout, committed to one
 //    mbarrier; every thread reads its row back with tcgen05.ld.
-// The CTA holds 128 tensor-memory columns (layer 2 at columns 0..63, layer 3
+// Each group holds 128 tensor-memory columns (layer 2 at columns 0..63, layer 3
 // at 64..79, or with the derivative chains of tile_eval_d: z2 0..63 and dz2
 // 64..127, then y 0..15 and dy 16..31).
 #pragma once
@@ -67,29 +68,88 @@ struct MlpDev {
   int nbins;
 };
 
+// The FP32 weights of tile_eval_d, a kernel parameter: every thread reads the
+// same one at a time, which from the constant bank costs no shared-memory
+// bandwidth (a broadcast load still delivers its bytes to all 32 lanes).
+struct __align__(16) MlpW {
+  float w1[NH], b1[NH], b2[NH];
+  float2 w3p[NH / 2][NO];  // W3 by pairs of hidden units: (W3[o][2q], W3[o][2q + 1])
+  float b3[NO];
+};
+inline void set_weights(MlpW &w, const float *par) {
+  for (int k = 0; k < NH; ++k) {
+    w.w1[k] = par[O_W1 + k];
+    w.b1[k] = par[O_B1 + k];
+    w.b2[k] = par[O_B2 + k];
+  }
+  for (int q = 0; q < NH / 2; ++q)
+    for (int o = 0; o < NO; ++o) w.w3p[q][o] = {par[O_W3 + o * NH + 2 * q], par[O_W3 + o * NH + 2 * q + 1]};
+  for (int o = 0; o < NO; ++o) w.b3[o] = par[O_B3 + o];
+}
+
+// Shared memory of a CTA of G groups of 128 threads, each with operand tiles,
+// a tensor-memory window and an mbarrier of its own; the weights are shared.
+// Four groups with the derivative tile fill an SM (221 KB, all 512
+// tensor-memory columns): 16 warps against 12 with three one-group CTAs.
+// NOPS operand tiles a group: the activations hi and lo and, for tile_eval_d,
+// the BF16 forward-mode derivative of the activations.
+template <int G_, int NOPS_>
 struct __align__(1024) Smem {
-  uint16_t a_hi[TILE * NH];  // 16 KB each
-  uint16_t a_lo[TILE * NH];
-  uint16_t w2_hi[NH * NH];   // 8 KB each
+  static constexpr int G = G_, NOPS = NOPS_;
+  uint16_t ops[G][NOPS][TILE * NH];  // 16 KB each
+  uint16_t w2_hi[NH * NH];           // 8 KB each
   uint16_t w2_lo[NH * NH];
-  uint16_t w3_hi[NOP * NH];  // 2 KB each
+  uint16_t w3_hi[NOP * NH];          // 2 KB each
   uint16_t w3_lo[NOP * NH];
-  alignas(16) float w1[NH];  // read as 16-byte vectors
+  alignas(16) float w1[NH];          // read as 16-byte vectors
   alignas(16) float b1[NH];
   alignas(16) float b2[NH];
   alignas(16) float b3[NOP];
   uint32_t gstep[kMaxGateBins / 32];  // bit b: bin b cleared for all of kStepMask
-  uint64_t bar;
+  uint64_t bar[G];
   uint32_t tmem;
-  int fail;
+  int fail[G];
 };
+using Smem1 = Smem<1, 2>;  // values only, one group, four CTAs per SM
+using SmemD = Smem<4, 3>;  // with the derivative, four groups, one CTA per SM (221 KB)
 
-// The same plus one BF16 operand tile for the forward-mode derivative of the
-// activations (tile_eval_d): 16 KB more, three CTAs per SM.
-struct __align__(1024) SmemD : Smem {
-  uint16_t d_hi[TILE * NH];
-  alignas(16) float2 w3p[NH / 2][NO];  // FP32 W3 by pairs of hidden units: (W3[o][2q], W3[o][2q + 1])
+// One group's view of the CTA: its thread's row of the tile, its tensor
+// memory and its index.
+struct Grp {
+  int r, g;
+  uint32_t tm;  // first tensor-memory column of the group
 };
+template <class S>
+__device__ __forceinline__ Grp grp_of(const S &s) {
+  const int g = threadIdx.x / TILE;
+  return {(int)threadIdx.x % TILE, g, s.tmem + (uint32_t)(TMEM_COLS * g)};
+}
+// Barrier over the group's 128 threads (barrier 0 is the CTA's; the warps are
+// converged first, the tensor-memory loads after it need whole warps).
+template <class S>
+__device__ __forceinline__ void grp_sync(const S &, const Grp &q) {
+  if constexpr (S::G == 1) {
+    __syncthreads();
+  } else {
+    __syncwarp();
+    asm volatile("barrier.sync %0, %1;" ::"r"(q.g + 1), "n"(TILE) : "memory");
+    __syncwarp();
+  }
+}
+// The same with the group's "or" of v.
+template <class S>
+__device__ __forceinline__ bool grp_or(const S &, const Grp &q, bool v) {
+  uint32_t any;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred p, o;\n\tsetp.ne.u32 p, %3, 0;\n\t"
+      "barrier.red.or.pred o, %1, %2, p;\n\tselp.u32 %0, 1, 0, o;\n\t}"
+      : "=r"(any)
+      : "r"(q.g + 1), "n"(TILE), "r"((uint32_t)v)
+      : "memory");
+  __syncwarp();
+  return any != 0;
+}
 
 // ---------------------------------------------------------------- PTX
 __device__ __forceinline__ float tanh_approx(float x) {
@@ -149,14 +209,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// 64 consecutive FP32 columns of this thread's TMEM lane in one load.
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float *v) {
+// Two runs of 32 columns under one wait.
+__device__ __forceinline__ void tmem_ld32x2(uint32_t ta, uint32_t tb, float *u, float *v) {
   uint32_t r[64];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,"
-      "%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,"
-      "%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%64];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%64];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,"
+      "%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%65];\n\t"
       "tcgen05.wait::ld.sync.aligned;"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
@@ -166,10 +226,13 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float *v) {
         "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]),
         "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
         "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
-      : "r"(taddr)
+      : "r"(ta), "r"(tb)
       : "memory");
 #pragma unroll
-  for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < 32; ++i) {
+    u[i] = __uint_as_float(r[i]);
+    v[i] = __uint_as_float(r[32 + i]);
+  }
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v) {
@@ -237,33 +300,36 @@ __device__ __forceinline__ void split2(uint64_t p, uint32_t &hi, uint32_t &lo) {
   lo = __byte_perm(__float_as_uint(l0), __float_as_uint(l1), 0x7632);
 }
 
-// Write one thread's 64 activations into row r of the hi and lo A tiles.
-__device__ __forceinline__ void store_split(Smem &s, int r, const float *a) {
+// Write 32 of a thread's activations into columns c0 .. c0 + 31 of row r of
+// the hi and lo operand tiles.
+__device__ __forceinline__ void store_split32(uint16_t *a_hi, uint16_t *a_lo, int r, int c0, const float *a) {
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
+  for (int c = 0; c < 4; ++c) {
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) split2(pk(a[8 * c + 2 * q], a[8 * c + 2 * q + 1]), hi[q], lo[q]);
-    const int off = tile_off(r, 8 * c);
-    *reinterpret_cast<uint4 *>(reinterpret_cast<char *>(s.a_hi) + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    *reinterpret_cast<uint4 *>(reinterpret_cast<char *>(s.a_lo) + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    const int off = tile_off(r, c0 + 8 * c);
+    *reinterpret_cast<uint4 *>(reinterpret_cast<char *>(a_hi) + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4 *>(reinterpret_cast<char *>(a_lo) + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
 }
 
 // The CTA's Smem inside its dynamic shared memory, placed on a 1024-byte
-// boundary (the kernels request sizeof(Smem) + 1024 bytes).
-template <class S = Smem>
+// boundary (the kernels request sizeof(S) + 1024 bytes).
+template <class S>
 __device__ __forceinline__ S &smem_of(unsigned char *raw) {
   const uint32_t a = smem_u32(raw);
   return *reinterpret_cast<S *>(raw + ((1024u - (a & 1023u)) & 1023u));
 }
-constexpr size_t kSmemBytes = sizeof(Smem) + 1024;
+constexpr size_t kSmemBytes = sizeof(Smem1) + 1024;
 constexpr size_t kSmemDBytes = sizeof(SmemD) + 1024;
+static_assert(kSmemDBytes <= 227 * 1024, "one CTA per SM");
 
 // ------------------------------------------------------------ CTA set-up
-// Load the weights into shared memory, initialise the mbarrier and allocate
-// the CTA's tensor memory (warp 0).  Every thread of the 128 calls it.
-__device__ __forceinline__ void cta_setup(Smem &s, const MlpDev &M) {
+// Load the weights into shared memory, initialise the mbarriers and allocate
+// the CTA's tensor memory (warp 0).  Every thread of the CTA calls it.
+template <class S>
+__device__ __forceinline__ void cta_setup(S &s, const MlpDev &M) {
   const int t = threadIdx.x;
   const uint4 *src = reinterpret_cast<const uint4 *>(M.wt);  // 16-byte aligned (host contract)
   uint4 *dst = reinterpret_cast<uint4 *>(s.w2_hi);  // w2_hi, w2_lo, w3_hi, w3_lo are contiguous
@@ -282,13 +348,15 @@ __device__ __forceinline__ void cta_setup(Smem &s, const MlpDev &M) {
     s.gstep[w] = bits;
   }
   if (t == 0) {
-    mbar_init(&s.bar, 1);
+    for (int g = 0; g < S::G; ++g) {
+      mbar_init(&s.bar[g], 1);
+      s.fail[g] = 0;
+    }
     chapsim::fence_mbar_init();
-    s.fail = 0;
   }
   if (t < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem)),
-                 "r"(TMEM_COLS)
+                 "r"(TMEM_COLS * S::G)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -298,27 +366,28 @@ __device__ __forceinline__ void cta_setup(Smem &s, const MlpDev &M) {
   tc_fence_after();
 }
 
-__device__ __forceinline__ void cta_teardown(Smem &s) {
+template <class S>
+__device__ __forceinline__ void cta_teardown(S &s) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (threadIdx.x < 32)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s.tmem), "r"(TMEM_COLS * S::G)
+                 : "memory");
 }
 
 // Issue one layer: D[:, 0:n) = A_hi W_hi^T + A_hi W_lo^T + A_lo W_hi^T over
-// K = 64 (four K = 16 steps each), then (commit) commit to the barrier.
-__device__ __forceinline__ void issue_layer(Smem &s, uint32_t dtm, const uint16_t *w_hi, const uint16_t *w_lo, int n,
-                                            bool commit = true) {
+// K = 64 (four K = 16 steps each).
+__device__ __forceinline__ void issue_layer(const uint16_t *a_hi, const uint16_t *a_lo, uint32_t dtm,
+                                            const uint16_t *w_hi, const uint16_t *w_lo, int n) {
   const uint32_t idesc = idesc_bf16(TILE, n);
-  const uint32_t ah = smem_u32(s.a_hi), al = smem_u32(s.a_lo), bh = smem_u32(w_hi), bl = smem_u32(w_lo);
+  const uint32_t ah = smem_u32(a_hi), al = smem_u32(a_lo), bh = smem_u32(w_hi), bl = smem_u32(w_lo);
   const uint32_t as[3] = {ah, ah, al}, bs[3] = {bh, bl, bh};
 #pragma unroll
   for (int part = 0; part < 3; ++part)
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks)
       umma(dtm, sdesc(as[part] + 256u * ks), sdesc(bs[part] + 256u * ks), idesc, (part | ks) ? 1u : 0u);
-  if (commit) umma_commit(&s.bar);
 }
 
 // One plain BF16 chain D[:, 0:n) = A W^T (K = 64) from the operand tiles a and w.
@@ -343,42 +412,44 @@ __device__ __forceinline__ void store_bf16_32(uint16_t *tile, int r, int c0, con
   }
 }
 
-// Block-uniform bounded wait for the layer's commit: false on every thread
+// Group-uniform bounded wait for the layer's commit: false on every thread
 // when any thread's wait ran out (the error word is set by mbar_wait).
-__device__ __forceinline__ bool layer_wait(Smem &s, uint32_t &phase, int *err) {
-  const bool ok = mbar_wait(&s.bar, phase, err);
+template <class S>
+__device__ __forceinline__ bool layer_wait(S &s, const Grp &q, uint32_t &phase, int *err) {
+  const bool ok = mbar_wait(&s.bar[q.g], phase, err);
   phase ^= 1u;
-  if (!ok) s.fail = 1;
-  __syncthreads();
+  if (!ok) s.fail[q.g] = 1;
+  grp_sync(s, q);
   tc_fence_after();
-  return s.fail == 0;
+  return s.fail[q.g] == 0;
 }
 
-// Layer 1 of one cell: a = tanh(w1 x + b1), the affine part on FP32 pairs.
-__device__ __forceinline__ void layer1(const Smem &s, float x, float (&a)[NH]) {
+// 32 units of layer 1 of one cell: a = tanh(w1 x + b1), the affine part on
+// FP32 pairs.
+__device__ __forceinline__ void layer1_32(const float *w1, const float *b1, float x, float *a) {
   const uint64_t xx = pk(x, x);
-  const uint4 *w = reinterpret_cast<const uint4 *>(s.w1), *b = reinterpret_cast<const uint4 *>(s.b1);
+  const uint4 *w = reinterpret_cast<const uint4 *>(w1), *b = reinterpret_cast<const uint4 *>(b1);
 #pragma unroll
-  for (int q = 0; q < NH / 4; ++q) {
+  for (int q = 0; q < 8; ++q) {
     const uint4 wq = w[q], bq = b[q];
     upk(fma2(pku(wq.x, wq.y), xx, pku(bq.x, bq.y)), a[4 * q], a[4 * q + 1]);
     upk(fma2(pku(wq.z, wq.w), xx, pku(bq.z, bq.w)), a[4 * q + 2], a[4 * q + 3]);
   }
 #pragma unroll
-  for (int k = 0; k < NH; ++k) a[k] = tanh_approx(a[k]);
+  for (int k = 0; k < 32; ++k) a[k] = tanh_approx(a[k]);
 }
 
-// a = tanh(a + bias) over the 64 hidden units, the adds on FP32 pairs.
-__device__ __forceinline__ void bias_tanh(const float *bias, float (&a)[NH]) {
+// a = tanh(a + bias) over 32 hidden units, the adds on FP32 pairs.
+__device__ __forceinline__ void bias_tanh32(const float *bias, float *a) {
   const uint4 *b = reinterpret_cast<const uint4 *>(bias);
 #pragma unroll
-  for (int q = 0; q < NH / 4; ++q) {
+  for (int q = 0; q < 8; ++q) {
     const uint4 bq = b[q];
     upk(add2(pk(a[4 * q], a[4 * q + 1]), pku(bq.x, bq.y)), a[4 * q], a[4 * q + 1]);
     upk(add2(pk(a[4 * q + 2], a[4 * q + 3]), pku(bq.z, bq.w)), a[4 * q + 2], a[4 * q + 3]);
   }
 #pragma unroll
-  for (int k = 0; k < NH; ++k) a[k] = tanh_approx(a[k]);
+  for (int k = 0; k < 32; ++k) a[k] = tanh_approx(a[k]);
 }
 
 // t[k] = (1 - a[k]^2) g[k] for 32 consecutive units, on FP32 pairs: the
@@ -391,49 +462,49 @@ __device__ __forceinline__ void dtanh32(const float *a, const float *g, float *t
   }
 }
 
-// cta_setup plus the FP32 layer-3 weights of tile_eval_d.
-__device__ __forceinline__ void cta_setup_d(SmemD &s, const MlpDev &M) {
-  for (int i = threadIdx.x; i < (NH / 2) * NO; i += blockDim.x) {
-    const int q = i / NO, o = i % NO;
-    s.w3p[q][o] = make_float2(M.par[O_W3 + o * NH + 2 * q], M.par[O_W3 + o * NH + 2 * q + 1]);
-  }
-  cta_setup(s, M);  // ends with a block barrier
-}
-
 // Evaluate the MLP on the tile: thread r holds cell r's normalised input x
 // and receives y[0..4] (standardised residual outputs, b3 included).  Every
-// thread of the CTA calls it together.  Returns false when a wait ran out
+// thread of the group calls it together.  Returns false when a wait ran out
 // (then y is not valid and the caller stops).
-__device__ __forceinline__ bool tile_eval(Smem &s, float x, float (&y)[NO], uint32_t &phase, int *err) {
-  const int r = threadIdx.x;
-  const uint32_t lane_base = s.tmem + ((uint32_t)(r & ~31) << 16);
-  float a[NH];
-  layer1(s, x, a);
-  store_split(s, r, a);
+template <class S>
+__device__ __forceinline__ bool tile_eval(S &s, const Grp &q, float x, float (&y)[NO], uint32_t &phase, int *err) {
+  uint16_t *a_hi = s.ops[q.g][0], *a_lo = s.ops[q.g][1];
+  const uint32_t lane_base = q.tm + ((uint32_t)(q.r & ~31) << 16);
+  float a[32];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    layer1_32(s.w1 + 32 * h, s.b1 + 32 * h, x, a);
+    store_split32(a_hi, a_lo, q.r, 32 * h, a);
+  }
   chapsim::fence_proxy_async();
   tc_fence_before();
-  __syncthreads();
-  if (r == 0) {
+  grp_sync(s, q);
+  if (q.r == 0) {
     tc_fence_after();
-    issue_layer(s, s.tmem, s.w2_hi, s.w2_lo, NH);
+    issue_layer(a_hi, a_lo, q.tm, s.w2_hi, s.w2_lo, NH);
+    umma_commit(&s.bar[q.g]);
   }
-  if (!layer_wait(s, phase, err)) return false;
-  tmem_ld64(lane_base, a);
-  bias_tanh(s.b2, a);
-  store_split(s, r, a);  // the layer-2 MMAs have completed: the A tiles are free
+  if (!layer_wait(s, q, phase, err)) return false;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {  // the layer-2 MMAs have completed: the A tiles are free
+    tmem_ld32(lane_base + 32 * h, a);
+    bias_tanh32(s.b2 + 32 * h, a);
+    store_split32(a_hi, a_lo, q.r, 32 * h, a);
+  }
   chapsim::fence_proxy_async();
   tc_fence_before();
-  __syncthreads();
-  if (r == 0) {
+  grp_sync(s, q);
+  if (q.r == 0) {
     tc_fence_after();
-    issue_layer(s, s.tmem + NH, s.w3_hi, s.w3_lo, NOP);
+    issue_layer(a_hi, a_lo, q.tm + NH, s.w3_hi, s.w3_lo, NOP);
+    umma_commit(&s.bar[q.g]);
   }
-  if (!layer_wait(s, phase, err)) return false;
+  if (!layer_wait(s, q, phase, err)) return false;
   float o[8];
   tmem_ld8(lane_base + NH, o);
 #pragma unroll
-  for (int q = 0; q < NO; ++q) y[q] = o[q] + s.b3[q];
-  tc_fence_before();  // the next tile's MMAs overwrite these columns after its first __syncthreads
+  for (int k = 0; k < NO; ++k) y[k] = o[k] + s.b3[k];
+  tc_fence_before();  // the next tile's MMAs overwrite these columns after its first group barrier
   return true;
 }
 
@@ -448,54 +519,50 @@ __device__ __forceinline__ bool tile_eval(Smem &s, float x, float (&y)[NO], uint
 // its MMAs but saves their round trip through shared memory, the tensor
 // pipe and tensor memory (one block barrier and one wait per tile), and its
 // FP32 products are more accurate than the split BF16 ones.  Tensor memory:
-// z2 in columns 0..63, dz2 in 64..127.  Every thread of the CTA calls it
-// together.  The layer-2 wait has no block barrier after it (nothing it
+// z2 in columns 0..63, dz2 in 64..127.  Every thread of the group calls it
+// together.  The layer-2 wait has no group barrier after it (nothing it
 // guards is shared: each thread reads its own tensor-memory lane after
 // seeing the commit itself); a wait that ran out sets s.fail, which the
-// caller reads after its next block barrier (the results are then
+// caller reads after its next group barrier (the results are then
 // discarded).
-__device__ __forceinline__ void tile_eval_d(SmemD &s, float x, float (&y)[NO], float (&dy)[NO], uint32_t &phase,
-                                            int *err) {
-  const int r = threadIdx.x;
-  const uint32_t lane_base = s.tmem + ((uint32_t)(r & ~31) << 16);
-  float a[NH];
-  layer1(s, x, a);
-  store_split(s, r, a);
+__device__ __forceinline__ void tile_eval_d(SmemD &s, const MlpW &W, const Grp &q, float x, float (&y)[NO],
+                                            float (&dy)[NO], uint32_t &phase, int *err) {
+  uint16_t *a_hi = s.ops[q.g][0], *a_lo = s.ops[q.g][1], *d_hi = s.ops[q.g][2];
+  const uint32_t lane_base = q.tm + ((uint32_t)(q.r & ~31) << 16);
+  float a[32], t[32];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    float t[32];
-    dtanh32(a + 32 * h, s.w1 + 32 * h, t);
-    store_bf16_32(s.d_hi, r, 32 * h, t);
+    layer1_32(W.w1 + 32 * h, W.b1 + 32 * h, x, a);
+    store_split32(a_hi, a_lo, q.r, 32 * h, a);
+    dtanh32(a, W.w1 + 32 * h, t);
+    store_bf16_32(d_hi, q.r, 32 * h, t);
   }
   chapsim::fence_proxy_async();
   tc_fence_before();
-  __syncthreads();
-  if (r == 0) {
+  grp_sync(s, q);
+  if (q.r == 0) {
     tc_fence_after();
-    issue_layer(s, s.tmem, s.w2_hi, s.w2_lo, NH, false);
-    issue_chain(s.tmem + NH, s.d_hi, s.w2_hi, NH);
-    umma_commit(&s.bar);
+    issue_layer(a_hi, a_lo, q.tm, s.w2_hi, s.w2_lo, NH);
+    issue_chain(q.tm + NH, d_hi, s.w2_hi, NH);
+    umma_commit(&s.bar[q.g]);
   }
-  if (!mbar_wait(&s.bar, phase, err)) s.fail = 1;
+  if (!mbar_wait(&s.bar[q.g], phase, err)) s.fail[q.g] = 1;
   phase ^= 1u;
   tc_fence_after();
-  tmem_ld64(lane_base, a);
-  bias_tanh(s.b2, a);
   uint64_t acc[NO], dacc[NO];
 #pragma unroll
   for (int o = 0; o < NO; ++o) acc[o] = dacc[o] = 0ull;  // (+0.0f, +0.0f)
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    float g[32];
-    tmem_ld32(lane_base + NH + 32 * h, g);
-    dtanh32(a + 32 * h, g, g);  // da2 for units 32 h .. 32 h + 31
+    tmem_ld32x2(lane_base + 32 * h, lane_base + NH + 32 * h, a, t);
+    bias_tanh32(W.b2 + 32 * h, a);
+    dtanh32(a, t, t);  // da2 for units 32 h .. 32 h + 31
 #pragma unroll
-    for (int qq = 0; qq < 16; ++qq) {
-      const int q = 16 * h + qq;
-      const uint64_t ap = pk(a[2 * q], a[2 * q + 1]), gp = pk(g[2 * qq], g[2 * qq + 1]);
+    for (int p = 0; p < 16; ++p) {
+      const uint64_t ap = pk(a[2 * p], a[2 * p + 1]), gp = pk(t[2 * p], t[2 * p + 1]);
 #pragma unroll
       for (int o = 0; o < NO; ++o) {
-        const uint64_t w = *reinterpret_cast<const uint64_t *>(&s.w3p[q][o]);
+        const uint64_t w = *reinterpret_cast<const uint64_t *>(&W.w3p[16 * h + p][o]);
         acc[o] = fma2(w, ap, acc[o]);
         dacc[o] = fma2(w, gp, dacc[o]);
       }
@@ -505,11 +572,11 @@ __device__ __forceinline__ void tile_eval_d(SmemD &s, float x, float (&y)[NO], f
   for (int o = 0; o < NO; ++o) {
     float e0, e1;
     upk(acc[o], e0, e1);
-    y[o] = (e0 + e1) + s.b3[o];
+    y[o] = (e0 + e1) + W.b3[o];
     upk(dacc[o], e0, e1);
     dy[o] = e0 + e1;
   }
-  tc_fence_before();  // the next tile's MMAs overwrite the columns read here after its first __syncthreads
+  tc_fence_before();  // the next tile's MMAs overwrite the columns read here after its first group barrier
 }
 
 // Largest step |x_new - x_old| over which a tile takes the properties at the
@@ -520,7 +587,7 @@ __device__ __forceinline__ void tile_eval_d(SmemD &s, float x, float (&y)[NO], f
 // model a second time.
 constexpr double kTaylorMax = 1e-3;
 
-// Assemble output o from the standardised residual y at input x (FP64).// Assemble output o from the standardised residual y at input x (FP64).
+// Assemble output o from the standardised residual y at input x (FP64).
 __device__ __forceinline__ double assemble(const MlpDev &M, int o, double x, float y) {
   double b = M.base[o][NBASE - 1];
 #pragma unroll
@@ -537,7 +604,8 @@ __device__ __forceinline__ unsigned gate_mask(const MlpDev &M, double h) { retur
 
 // Whether the gate cleared h's bin for every output of kStepMask (the CTA's
 // shared-memory copy of the gate, one bit per bin).
-__device__ __forceinline__ bool gate_step(const Smem &s, const MlpDev &M, double h) {
+template <class S>
+__device__ __forceinline__ bool gate_step(const S &s, const MlpDev &M, double h) {
   const int bin = gate_bin(M, h);
   return (s.gstep[bin >> 5] >> (bin & 31)) & 1u;
 }

@@ -84,9 +84,10 @@ __global__ void __launch_bounds__(chapsim_mlp::TILE, 4)
     k_props_mlp_tc(PropsDev P, const double *__restrict__ h, double *T, double *rho, double *mu, double *kk,
                    double *cp, int64_t n) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  chapsim_mlp::Smem &s = chapsim_mlp::smem_of(smem_raw);
+  chapsim_mlp::Smem1 &s = chapsim_mlp::smem_of<chapsim_mlp::Smem1>(smem_raw);
   const chapsim_mlp::MlpDev &M = P.M;
   chapsim_mlp::cta_setup(s, M);
+  const chapsim_mlp::Grp grp = chapsim_mlp::grp_of(s);
   uint32_t phase = 0;
   const int64_t ntiles = (n + chapsim_mlp::TILE - 1) / chapsim_mlp::TILE;
   const unsigned need = cp ? 0x1Fu : chapsim_mlp::kStepMask;
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(chapsim_mlp::TILE, 4)
     const double hv = c < n ? h[c] : 0.0;
     const double x = (hv - M.hmid) / M.hhalf;
     float y[NO];
-    if (!chapsim_mlp::tile_eval(s, (float)x, y, phase, P.dev_err)) break;
+    if (!chapsim_mlp::tile_eval(s, grp, (float)x, y, phase, P.dev_err)) break;
     if (c >= n || fabs(hv) < 1.0e-10) continue;  // reference leaves these cells unchanged
     if (!(hv > P.ht.x[0] && hv < P.ht.x[P.ht.n - 1])) {
       atomicAdd(P.err_count, 1);

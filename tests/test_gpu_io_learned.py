@@ -158,3 +158,41 @@ def test_therm_prop_update_learned_vs_table(table, engine):
     g.therm_prop_update(mode=1)
     for n, r in ref.items():
         assert relerr(g.get_field(n)[:, 1:-1, :], r) <= 2e-4, n
+
+
+@pytest.mark.parametrize("far", [False, True], ids=["near", "far"])
+@pytest.mark.parametrize("dims", [(20, 6, 12), (40, 18, 24), (50, 20, 36), (96, 46, 64)],
+                         ids=lambda d: "x".join(map(str, d)))
+def test_energy_substep_properties_are_the_models_at_its_enthalpy(table, engine, dims, far):
+    """The properties an energy substep leaves against the model evaluated
+    anew at the enthalpy it leaves, from fewer tiles than blocks over one
+    tile more than a round to several tiles a group with a ragged last one.
+    near: one evaluation and its first-order expansion (dropped term below
+    1e-5 of a property's range, derivative chain and both roundings below
+    that): 1e-4 as the gate.  far: densities 5 % off, so steps far beyond the
+    expansion's limit; both sides evaluate the same layers, the inputs' FP32
+    rounding (6e-8) apart: 1e-6."""
+    from chapsim1ww_b200 import IOChannel, _lib
+    g = IOChannel(*dims, table=table)
+    g.set_props_mode(_lib.PROPS_MLP, engine)
+    g.random_fl_theml_fld_io(3, 0.1)
+    h = g.get_field("h")
+    z, y, x = np.meshgrid(*(np.linspace(0, 2 * np.pi, n, endpoint=False) for n in h.shape), indexing="ij")
+    h[:, 1:-1, :] = (0.3 + 0.2 * np.sin(x) * np.cos(y) * np.cos(z))[:, 1:-1, :]
+    g.set_field("h", h)
+    g.therm_prop_update(mode=0)
+    rho = g.get_field("rho")
+    g.set_field("rhoh", rho * h)
+    if far:
+        g.set_field("rho", rho * np.random.default_rng(5).uniform(0.95, 1.05, rho.shape))
+    before = g.model_again_tiles()
+    g.solverrk3_eng_io(1)
+    again = g.model_again_tiles() - before
+    cells = dims[0] * (dims[1] + 2) * dims[2]
+    assert again >= (cells // 128 if far else 0)
+    got = {n: g.get_field(n)[:, 1:-1, :] for n in ("t", "rho", "mu", "k")}
+    assert g.bad_cells() == 0
+    g.therm_prop_update(mode=1)
+    for n, v in got.items():
+        ref = g.get_field(n)[:, 1:-1, :]
+        assert relerr(v, ref) <= (1e-6 if far else 1e-4), n
