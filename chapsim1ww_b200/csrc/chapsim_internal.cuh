@@ -226,6 +226,7 @@ struct chapsim_ctx {
   cudaGraphExec_t io_graph[2] = {nullptr, nullptr};  // one step starting from io_cur = 0 / 1
   // TMA descriptors of the IO momentum RHS: u, v, w, p, mu0 + mu, g[0][0..2], g[1][0..2], EXPLT0
   CUtensorMap io_maps[14];
+  CUtensorMap eng_maps[3];  // energy equation: h, T, k
   CUtensorMap si_maps[4];  // semi-implicit scheme: mu, DRHOI_STG 1-3
   bool use_tma_si = false;
   bool use_tma_io = false;

@@ -130,7 +130,10 @@ struct Look {
 
 // ---------------------------------------------------------------- energy
 // RHS_ENERGY_EXPLICIT and the RHOH update of SOLVERRK3_ENG_IO (:22-35):
-// rhoh += gam dt R + zeta dt R_old, limited to RHOHmax + REALMIN.  Six blocks
+// rhoh += gam dt R + zeta dt R_old, limited to RHOHmax + REALMIN.  This form,
+// one cell per thread, serves grids too small for the TMA boxes and the mixed
+// form (whose FP32 Poisson solve magnifies a change of the last bits); the
+// others take k_io_eng_rhs_tma.  Six blocks
 // per SM (40 registers): latency-bound on its neighbour loads, it gains from
 // the extra resident warps (measured 0.536 -> 0.510 ms at 512x192x256).
 __global__ void __launch_bounds__(IO_BX *IO_BY, 6) k_io_eng_rhs(TGDev d, IODev io, double cdt1, double cdt0, int cur) {
@@ -826,6 +829,9 @@ constexpr size_t IT_SLOT = (size_t)IT_NF * IT_PST * sizeof(double);
 constexpr size_t IT_ESLOT = (size_t)3 * IT_EBOX * sizeof(double);
 static_assert((IT_PST * 8) % 128 == 0 && IT_PST >= IT_PLANE, "TMA destinations must stay 128-byte aligned");
 static_assert(IT_SLOT % 128 == 0 && IT_ESLOT % 128 == 0 && (IT_EBOX * 8) % 128 == 0, "128-byte aligned slots");
+struct EngMaps {
+  CUtensorMap m[7];  // h, T, k, G x, G0 x, G y, G0 y
+};
 struct IoMaps {
   CUtensorMap m[14];  // u, v, w, p, msum, g[0][0..2], g[1][0..2], EXPLT0[0..2]
 };
@@ -852,6 +858,149 @@ template <bool CPL> struct ItGeo {
 static_assert((ItGeo<true>::PST * 8) % 128 == 0 && ItGeo<true>::PST >= ItGeo<true>::PLANE &&
                   (ItGeo<true>::BXW * 8) % 16 == 0,
               "coupled TMA boxes: 128-byte aligned destinations, 16-byte rows");
+
+// k_io_eng_rhs as a march along z over nzc planes of a 32 x 8 (x, y) tile.
+// h, T, k and the x and y components of G and G0 arrive as TMA boxes (as in
+// k_io_rhs_tma below) in a ring of three plane slots: plane k for the x and y
+// neighbours, plane k + 1 for the column ahead, plane k + 2 in flight; the
+// plane behind and the z fluxes stay in registers.  62 KB let three blocks
+// share a multiprocessor.  The kernel of one cell per thread issues 37 loads
+// and waits for them (DRAM 48 %): 0.351 -> 0.275 ms at 384x192x192, 0.615 ->
+// 0.446 at 512x192x256 coupled, 16.5 -> 15.7 us at 100x49x60; its bytes take
+// 0.228 ms at 384x192x192.  16 planes a block: 0.275 at 8, 0.279 at 32, 0.308
+// at 64 (the planes of many long marches fall out of L2 between tiles).
+constexpr int ET_NF = 7, E_H = 0, E_T = 1, E_K = 2, E_GX = 3, E_HX = 4, E_GY = 5, E_HY = 6;
+template <bool CPL> constexpr size_t et_smem() {
+  return (size_t)3 * ET_NF * ItGeo<CPL>::PST * sizeof(double) + 3 * sizeof(uint64_t);
+}
+
+template <bool CPL>
+__global__ void __launch_bounds__(IO_BX *IO_BY, 3)
+k_io_eng_rhs_tma(const __grid_constant__ EngMaps maps, TGDev d, IODev io, double cdt1, double cdt0, int cur, int nzc) {
+  typedef ItGeo<CPL> G;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  double *ring = reinterpret_cast<double *>(smem_raw);
+  auto slot = [&](int sl) { return ring + (size_t)sl * ET_NF * G::PST; };
+  uint64_t *bar = reinterpret_cast<uint64_t *>(ring + (size_t)3 * ET_NF * G::PST);
+  __shared__ const double *src[ET_NF];
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + IO_BX * ty;
+  const int x0 = blockIdx.x * IO_BX, j0 = 1 + blockIdx.y * IO_BY;
+  const int kbeg = blockIdx.z * nzc, kend = min(kbeg + nzc, nz);
+  const int i = x0 + tx, j = j0 + ty;
+  const bool active = i < nx && j <= ny;
+  const bool left_edge = x0 == 0, right_edge = x0 + IO_BX >= nx;
+  const int right_col = nx - x0 + 2;  // smem column of x = nx (wraps to 0)
+  const double *__restrict__ gz = io.g[cur][2], *__restrict__ hz = io.g[1 - cur][2];
+  if (tid == 0) {
+    for (int q = 0; q < 3; ++q) mbar_init(&bar[q], 1);
+    fence_mbar_init();
+    const double *f[ET_NF] = {io.h, io.T, io.kap, io.g[cur][0], io.g[1 - cur][0], io.g[cur][1], io.g[1 - cur][1]};
+    for (int q = 0; q < ET_NF; ++q) src[q] = f[q];
+  }
+  __syncthreads();
+  auto wrap = [&](int k) { return k < 0 ? k + nz : (k >= nz ? k - nz : k); };
+  auto issue = [&](int k, int sl) {
+    mbar_expect_tx(&bar[sl], (uint32_t)(ET_NF * G::PLANE * sizeof(double)));
+#pragma unroll
+    for (int f = 0; f < ET_NF; ++f) tma_load_3d(slot(sl) + f * G::PST, &maps.m[f], x0 - 2, j0 - 1, wrap(k), &bar[sl]);
+  };
+  uint32_t par = 0;
+  auto wait_plane = [&](int k, int sl) -> bool {
+    const bool ok = mbar_wait(&bar[sl], (par >> sl) & 1u, d.err);
+    par ^= 1u << sl;
+    if (CPL) return ok;  // the coupled section's ghost columns came with the box
+    if (left_edge && tid < 10 * ET_NF) {
+      const int f = tid / 10, r = tid - f * 10, jr = j0 - 1 + r;
+      if (jr <= ny + 1) slot(sl)[f * G::PST + r * G::BXW + 1] = src[f][(nx - 1) + d.sy * jr + d.sz * wrap(k)];
+    }
+    if (right_edge && tid >= 128 && tid < 128 + 10 * ET_NF) {
+      const int q = tid - 128, f = q / 10, r = q - f * 10, jr = j0 - 1 + r;
+      if (jr <= ny + 1) slot(sl)[f * G::PST + r * G::BXW + right_col] = src[f][d.sy * jr + d.sz * wrap(k)];
+    }
+    return ok;
+  };
+  if (tid == 0) {
+    issue(kbeg, 0);
+    issue(kbeg + 1, 1);
+  }
+  const double coe1 = d.dxi * 0.5 * 0.5, coe11 = d.dxqi * 0.5 * io.cthecd, coe3 = d.dzi * 0.5 * 0.5;
+  const double coe33 = d.dzqi * 0.5 * io.cthecd;
+  const bool iso_bot = io.isothermal & 1, iso_top = io.isothermal & 2;
+  double coe2 = 0.0, coe22 = 0.0, coe221 = 0.0, coe222 = 0.0, wffp = 0.0, wfbp = 0.0, wff = 0.0, wfb = 0.0;
+  // the cell's own column: the plane behind (h, T, k), the z fluxes' G + G0
+  double hm = 0.0, tm = 0.0, km = 0.0, az = 0.0;
+  if (active) {
+    coe2 = d.dyfi[j] * 0.5;
+    coe22 = d.dyfi[j] * io.cthecd;
+    coe221 = j == ny && !iso_top ? 1.0 : d.dyci[j + 1];  // iso-flux wall rows as in k_io_eng_rhs
+    coe222 = j == 1 && !iso_bot ? 1.0 : d.dyci[j];
+    wffp = d.wff[j + 1];
+    wfbp = d.wfb[j + 1];
+    wff = d.wff[j];
+    wfb = d.wfb[j];
+    const int64_t cb = i + d.sy * j, cm = cb + d.sz * wrap(kbeg - 1), cc = cb + d.sz * kbeg;
+    hm = io.h[cm];
+    tm = io.T[cm];
+    km = io.kap[cm];
+    az = hz[cc] + gz[cc];
+  }
+  bool ok = wait_plane(kbeg, 0);
+  int sl = 0;  // plane k's slot
+  const int at0 = (ty + 1) * G::BXW + tx + G::XO;
+  for (int k = kbeg; k < kend; ++k) {
+    const int64_t c = i + d.sy * j + d.sz * k, cp = i + d.sy * j + d.sz * wrap(k + 1);
+    double rh = 0.0, r0 = 0.0, azp = 0.0;
+    if (active) {  // hides behind the plane wait
+      rh = io.rhoh[c];
+      r0 = io.rhse0[c];
+      azp = hz[cp] + gz[cp];
+    }
+    const int sp = sl == 2 ? 0 : sl + 1, sn = sp == 2 ? 0 : sp + 1;
+    ok = wait_plane(k + 1, sp) && ok;
+    __syncthreads();  // plane k + 1 is complete, plane k - 1 no longer read
+    if (tid == 0 && k + 2 <= kend) {
+      fence_proxy_async();
+      issue(k + 2, sn);
+    }
+    if (active && ok) {
+      const double *S = slot(sl) + at0, *Sp = slot(sp) + at0;
+#define A(f, dx, dy) S[(f) * G::PST + (dy) * G::BXW + (dx)]
+      const double hc = A(E_H, 0, 0), hp = Sp[E_H * G::PST];
+      double dx_rhohu = (A(E_H, 1, 0) + hc) * (A(E_HX, 1, 0) + A(E_GX, 1, 0)) -
+                        (hc + A(E_H, -1, 0)) * (A(E_HX, 0, 0) + A(E_GX, 0, 0));
+      dx_rhohu *= coe1;
+      double dy_rhohv = (wffp * A(E_H, 0, 1) + wfbp * hc) * (A(E_HY, 0, 1) + A(E_GY, 0, 1)) -
+                        (wff * hc + wfb * A(E_H, 0, -1)) * (A(E_HY, 0, 0) + A(E_GY, 0, 0));
+      dy_rhohv *= coe2;
+      double dz_rhohw = (hp + hc) * azp - (hc + hm) * az;
+      dz_rhohw *= coe3;
+      const double tc = A(E_T, 0, 0), kc = A(E_K, 0, 0), tp = Sp[E_T * G::PST], kp = Sp[E_K * G::PST];
+      double dx_kdt = (A(E_K, 1, 0) + kc) * (A(E_T, 1, 0) - tc) - (kc + A(E_K, -1, 0)) * (tc - A(E_T, -1, 0));
+      dx_kdt *= coe11;
+      double kdty1 = (wffp * A(E_K, 0, 1) + wfbp * kc) * (A(E_T, 0, 1) - tc) * coe221;
+      double kdty2 = (wff * kc + wfb * A(E_K, 0, -1)) * (tc - A(E_T, 0, -1)) * coe222;
+#undef A
+      if (j == 1 && !iso_bot)
+        kdty2 = -io.qw_bot * coe222;  // WALLFLUX(bottom) = +qw
+      else if (j == ny && !iso_top)
+        kdty1 = io.qw_top * coe221;   // -WALLFLUX(top), WALLFLUX(top) = -qw
+      const double dy_kdt = (kdty1 - kdty2) * coe22;
+      double dz_kdt = (kp + kc) * (tp - tc) - (km + kc) * (tc - tm);
+      dz_kdt *= coe33;
+      const double R = -dx_rhohu - dy_rhohv - dz_rhohw + dx_kdt + dy_kdt + dz_kdt;
+      double r = rh + cdt1 * R + cdt0 * r0;
+      r = fmin(io.rhohmax + 1.0e-14, r);
+      io.rhoh[c] = r;
+      io.rhse0[c] = R;
+      hm = hc;
+      tm = tc;
+      km = kc;
+      az = azp;
+    }
+    sl = sp;
+  }
+}
 
 template <bool TH, bool CPL>
 __global__ void __launch_bounds__(IO_BX *IO_BY, 2)
@@ -1327,7 +1476,26 @@ int io_eng(chapsim_ctx *c, int ns) {
   TGDev &d = c->d;
   const SubParams &sp = c->sp[ns];
   phase_mark(c, 0);
-  k_io_eng_rhs<<<cell_grid(d), dim3(IO_BX, IO_BY), 0, c->stream>>>(d, c->io, sp.gam * d.dt, sp.roh * d.dt, c->io_cur);
+  const dim3 grid = cell_grid(d), blk(IO_BX, IO_BY);
+  if (c->use_tma_io && c->cfg.precision != CHAPSIM_MIXED) {
+    EngMaps maps;
+    const int cur = c->io_cur;
+    memcpy(maps.m, c->eng_maps, sizeof(c->eng_maps));
+    for (int q = 0; q < 2; ++q) {
+      maps.m[E_GX + 2 * q] = c->io_maps[5 + 3 * cur + q];
+      maps.m[E_HX + 2 * q] = c->io_maps[5 + 3 * (1 - cur) + q];
+    }
+    const int nzc = march_len((int64_t)grid.x * grid.y, d.nz, 16, 4, 2 * c->nsm);
+    const dim3 g3(grid.x, grid.y, (d.nz + nzc - 1) / nzc);
+    if (c->xnp)
+      k_io_eng_rhs_tma<true><<<g3, blk, et_smem<true>(), c->stream>>>(maps, d, c->io, sp.gam * d.dt, sp.roh * d.dt,
+                                                                       cur, nzc);
+    else
+      k_io_eng_rhs_tma<false><<<g3, blk, et_smem<false>(), c->stream>>>(maps, d, c->io, sp.gam * d.dt, sp.roh * d.dt,
+                                                                         cur, nzc);
+  } else {
+    k_io_eng_rhs<<<grid, blk, 0, c->stream>>>(d, c->io, sp.gam * d.dt, sp.roh * d.dt, c->io_cur);
+  }
   LAUNCHED();
   dim3 g2((d.nx + IO_BX - 1) / IO_BX, (d.ny + 2 + IO_BY - 1) / IO_BY, d.nz);
   phase_mark(c, 1);
@@ -1468,6 +1636,19 @@ int io_init_maps(chapsim_ctx *c) {
       c->err = "cuTensorMapEncodeTiled failed";
       return CHAPSIM_ERR_CUDA;
     }
+  }
+  if (io.thermal) {
+    void *fe[3] = {io.h - xo, io.T - xo, io.kap - xo};
+    for (int m = 0; m < 3; ++m)
+      if (encode(&c->eng_maps[m], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, fe[m], dims, strides, box, es,
+                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+        c->err = "cuTensorMapEncodeTiled failed";
+        return CHAPSIM_ERR_CUDA;
+      }
+    const void *fn = cpl ? (const void *)k_io_eng_rhs_tma<true> : (const void *)k_io_eng_rhs_tma<false>;
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)(cpl ? et_smem<true>() : et_smem<false>())));
   }
   if (io.visc) {
     void *fs[4] = {io.mu, io.drhoi[0], io.drhoi[1], io.drhoi[2]};

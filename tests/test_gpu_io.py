@@ -333,3 +333,23 @@ def test_io_substep_calls_replay_the_same_launches_bitwise(visc):
         b.step(7)
         for f in FLOW + THERMAL + ("g0x", "rho0"):
             assert np.array_equal(a.get_field(f), b.get_field(f)), f
+
+
+@pytest.mark.parametrize("dims", [(36, 8, 8), (50, 9, 10), (64, 16, 18), (66, 17, 40), (160, 96, 50)],
+                         ids=lambda d: "x".join(map(str, d)))
+def test_energy_rhs_march_edges(dims):
+    """Energy substeps on grids whose last tile or last march is short (one
+    to sixteen planes a block, the wrap in z, the patched x columns), with an
+    enthalpy and mass fluxes that vary in every direction."""
+    g, o = pair(*dims, thermal=1)
+    rng = np.random.default_rng(11)
+    rhoh = 0.3 * rng.uniform(-1.0, 1.0, g.shape)
+    T = 1.0 + 0.2 * rng.uniform(-1.0, 1.0, g.shape)
+    for x, put in ((g, g.set_field), (o, o.set)):
+        put("h", rhoh)
+        put("t", T)
+        put("rhoh", rhoh)
+    for ns in (1, 2):
+        g.solverrk3_eng_io(ns)
+        o.eng(ns)
+        compare(g, o, THERMAL, tag=f"eng{ns}")
