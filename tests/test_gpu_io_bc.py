@@ -113,3 +113,23 @@ def test_boundary_operator_errors():
         io.bc_coutlet_mom_rk3(4)
     with pytest.raises(ValueError):
         io.set_plane("out_u", np.zeros(3))
+
+
+@pytest.mark.parametrize("ny,nz", [(31, 32), (33, 64), (64, 128), (91, 200)])
+def test_outlet_reductions_over_the_plane(ny, nz):
+    """The outlet velocity range and the mass balance on planes of less than
+    one block of threads up to more than two values a thread, with a ragged
+    remainder, and partial sums in both regimes."""
+    tg, g, o = _setup(16, 40, ny, nz)
+    g.bc_tinlet_flow(tg)
+    o.bc_tinlet_flow(*(tg.get_field(n) for n in ("u", "v", "w", "p")))
+    g.bc_coutlet_mom_rk3(1)
+    o.bc_coutlet_mom_rk3(1)
+    g.bc_coutlet_eneg_rk3(1)
+    o.bc_coutlet_eneg_rk3(1)
+    sg, so = g.bc_scalars(), o.bc_scalars()
+    for key in ("u_outlet", "u_outlet_eng", "scaling", "inflow", "outflow"):
+        assert abs(sg[key] - so[key]) <= TOL * abs(so[key]), (key, sg[key], so[key])
+    # sums that cancel: against the size of what is summed
+    for key in ("mass_rate", "balance"):
+        assert abs(sg[key] - so[key]) <= TOL * abs(so["inflow"]), (key, sg[key], so[key])
