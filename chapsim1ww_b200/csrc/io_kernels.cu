@@ -1109,18 +1109,25 @@ k_io_rhs_tma(const __grid_constant__ IoMaps maps, TGDev d, IODev io, double gam,
 #pragma unroll
       for (int q = 0; q < 3; ++q) e0r[q] = ((const double *)d.h0[q])[ce];
     }
-    if (tid == 0) {
-      fence_proxy_async();
-      if (k + 2 <= kend) issue(k + 2);
-      if (!G::EREG && k + 1 < kend) issue_e(k + 1);
-    }
     ok = wait_plane(k + 1) && ok;
     if (!G::EREG) {
       const int esl = (k - kbeg) & 1;
       ok = mbar_wait(&ebar[esl], (epar >> esl) & 1u, d.err) && ok;
       epar ^= 1u << esl;
     }
+    // the plane's one barrier: plane k + 1 is complete, and every warp is done
+    // with the cells of plane k - 1, so the slot of plane k - 2 takes plane
+    // k + 2.  With a second barrier at the loop's end and the copy issued
+    // ahead of the wait: 0.536 against 0.518 ms at 384x192x192, 3.52 against
+    // 3.38 at 1024x384x256, 0.997 against 0.938 at 512x192x256 coupled (the
+    // TG kernel, whose planes take half the time, keeps that form: 0.267
+    // against 0.287 ms)
     __syncthreads();
+    if (tid == 0) {
+      fence_proxy_async();
+      if (k + 2 <= kend) issue(k + 2);
+      if (!G::EREG && k + 1 < kend) issue_e(k + 1);
+    }
     const double *Es = eslot((k - kbeg) & 1);
     if (active && ok) {
       const double *Sm = slot(slot_of(k - 1));
@@ -1295,7 +1302,6 @@ k_io_rhs_tma(const __grid_constant__ IoMaps maps, TGDev d, IODev io, double gam,
       }
 #undef A
     }
-    __syncthreads();
   }
   // every issued plane has been waited for, so no bulk copy is in flight at exit
   for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);

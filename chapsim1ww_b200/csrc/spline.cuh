@@ -42,7 +42,6 @@ __device__ __forceinline__ double spline_at(const Spline &s, int i, double u) {
   const double dx = u - __ldg(s.x + i);
   return r.x + dx * (r.y + dx * (r.z + dx * r.w));
 }
-__device__ __forceinline__ double spline_eval(const Spline &s, double u) { return spline_at(s, spline_find(s, u), u); }
 
 // ---------------------------------------------------------------- IO tables
 // The table of an IO context, laid out for look-ups by a warp of cells whose
