@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(SI_BX *SI_BY, 4) k_io_rhs_si(TGDev d, IODev io
 // the warps hide each other's shared-memory latency.  The per-component
 // kernels above read up to fourteen arrays from global memory, 60 loads per
 // cell and component, and wait for them (DRAM 17 %): 3.15 ms for the three at
-// 384x192x192 with the energy equation, 1.10 ms here (its bytes: 0.37 ms;
+// 384x192x192 with the energy equation, 1.00 ms here (its bytes: 0.37 ms;
 // shared-memory pipe 62 %, FP64 pipe 31 % busy).
 constexpr int ST_BXW = 36, ST_BYW = 10, ST_PLANE = ST_BXW * ST_BYW, ST_PST = 368;
 constexpr int S_U = 0, S_V = 1, S_W = 2, S_GX = 3, S_GY = 4, S_GZ = 5, S_P = 6, S_MU = 7, S_M = 8, S_R = 9;
