@@ -824,10 +824,12 @@ __global__ void __launch_bounds__(AY_TX *AY_TY) k_adiy_band(TGDev d, SubParams s
     const int r = t / GS, m = t - r * GS - W, j = min(j0 + r, ny);
     gsh[t] = m <= W ? sp.yg[comp][(size_t)j * (2 * AYB_WMAX + 1) + AYB_WMAX + m] : 0.0;
   }
-  // rows that no copy fills stay zero
+  // rows that no copy fills stay zero; row 1 of the v lines is left out of the
+  // FP64 form's fill: warp 0 stores it for every plane (all 32 columns), for
+  // the first one with no barrier in between
   for (int t = tid; t < AY_PD * TS; t += AY_TX * AY_TY) {
     const int row = t % TS / AY_TX, j = j0 - W + row;
-    if (row == NR || j < 1 || j > ny || (row1 && row == W)) ring[t] = (T)0;
+    if (row == NR || j < 1 || j > ny || (APART && row1 && row == W)) ring[t] = (T)0;
   }
   int kc = kb, cslot = 0;
   auto copy = [&]() {  // queue plane kc (an empty group past the end)

@@ -339,3 +339,23 @@ def test_x_transform_lengths(nx):
     g.solverrk3_mom_tg(0)
     o.substep(0)
     compare(g, o, tag=f"nx {nx}")
+
+
+# compiled widths 2, 4, 6 and 12 of the y factors: rows of the ring that
+# different warps clear
+@pytest.mark.parametrize("dt,ren", [(1e-5, 2800.0), (1e-3, 2800.0), (2e-2, 2800.0), (2e-2, 100.0)])
+def test_adi_first_plane_of_a_march(dt, ren):
+    """The v rows at the lower wall, which take the u increment of row 1, on
+    every plane (the first of each march of the y factors among them), over
+    several x tiles and repeated substeps; the same bits on a second run."""
+    runs = []
+    for _ in range(2):
+        g, o = pair(160, 36, 40, ren=ren, dt=dt, seed=6)
+        for ns in (0, 1, 2, 3):
+            g.solverrk3_mom_tg(ns)
+            o.substep(ns)
+            v, ref = g.get_field("v"), o.get("v")
+            err = np.abs(v - ref)[:, :18, :].max(axis=(1, 2)) / np.abs(ref).max()
+            assert (err <= TOL).all(), (ns, np.flatnonzero(err > TOL), err.max())
+        runs.append(v)
+    assert np.array_equal(*runs)
