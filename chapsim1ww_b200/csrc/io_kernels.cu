@@ -1415,8 +1415,14 @@ __global__ void __launch_bounds__(IO_BX *IO_BY) k_io_red_part(TGDev d, IODev io,
 // plane values), 97 -> 14 us for the mass balance (the planes and 98,304
 // partials, in one launch instead of two); the step alone 15.9 -> 15.6 ms.
 constexpr int RED_CL = 8;
+// A block may write another block's shared memory only once that block has
+// started.  Every thread arrives at the cluster's barrier here, first thing in
+// the kernel; cluster_reduce waits for it just before that write, so that the
+// loads in between hide it.
+__device__ __forceinline__ void cluster_start() { cooperative_groups::this_cluster().barrier_arrive(); }
 // Combine each thread's N values over the cluster in a fixed order: true on
-// the one thread that then holds the results.
+// the one thread that then holds the results.  Every thread of the cluster
+// calls cluster_start before and this after.
 template <int N, class Op>
 __device__ __forceinline__ bool cluster_reduce(double (&v)[N], Op op) {
   __shared__ double sw[N][32], sc[N][RED_CL];
@@ -1429,6 +1435,7 @@ __device__ __forceinline__ bool cluster_reduce(double (&v)[N], Op op) {
     if ((threadIdx.x & 31) == 0) sw[q][threadIdx.x >> 5] = v[q];
   }
   __syncthreads();
+  cl.barrier_wait();
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int q = 0; q < N; ++q) {
@@ -1447,6 +1454,7 @@ __device__ __forceinline__ bool cluster_reduce(double (&v)[N], Op op) {
 }
 
 __global__ void __cluster_dims__(RED_CL) __launch_bounds__(1024) k_io_red_final(TGDev d, int what, int npart) {
+  cluster_start();
   const bool mx = what != 1;
   double v[1] = {0.0};
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npart; t += RED_CL * blockDim.x)
@@ -1800,6 +1808,7 @@ __global__ void k_bc_inlet(TGDev d, IODev io, const double *__restrict__ tu, con
 // CONVCTION_OUTLET_U (src/BC_COUTLET_MOM_RK3.f90:101-174): (max + min) / 2 of
 // the outlet-face mean 0.5 (u(NCL1) + u(NCL1 + 1)) over j = 1..ny; one cluster.
 __global__ void __cluster_dims__(RED_CL) __launch_bounds__(1024) k_bc_umax(TGDev d, IODev io, int slot) {
+  cluster_start();
   const int nx = d.nx, ny = d.ny;
   const double *uo = bplane(io, CHAPSIM_P_OUT_U);
   double v[2] = {-1.0e20, 1.0e20};
@@ -1840,6 +1849,7 @@ __global__ void k_bc_outlet_conv(TGDev d, IODev io, double gam, double roh, int 
 // outflow from the planes and the mass rate from the npart block sums of
 // DrhoDtP / DYFI, each in a fixed order; one cluster.
 __global__ void __cluster_dims__(RED_CL) __launch_bounds__(1024) k_bc_mass(TGDev d, IODev io, int cur, int npart) {
+  cluster_start();
   const int ny = d.ny, t0 = blockIdx.x * blockDim.x + threadIdx.x, dt = RED_CL * blockDim.x;
   const double *go = bplane(io, CHAPSIM_P_OUT_GX);
   double v[3] = {0.0, 0.0, 0.0};  // inflow, outflow, mass rate
