@@ -1726,7 +1726,6 @@ int chapsim_phase_reset(chapsim_ctx *ctx) {
 int chapsim_set_tuning(chapsim_ctx *ctx, int rhs_nzc, int fft_lb) {
   if (!ctx || rhs_nzc < 1 || fft_lb < 0 || fft_lb > 64 || (fft_lb & 1)) return CHAPSIM_ERR_ARG;
   ctx->rhs_nzc = rhs_nzc;
-  ctx->io_nzc = rhs_nzc;  // the IO momentum RHS marches the same way
   ctx->nzc_set = true;
   ctx->fft_lb = fft_lb;
   drop_graphs(ctx);
@@ -1748,7 +1747,7 @@ int chapsim_get_line_tuning(const chapsim_ctx *ctx, int *ysolve_bx) {
 
 int chapsim_get_tuning(const chapsim_ctx *ctx, int *rhs_nzc, int *fft_lb) {
   if (!ctx || !rhs_nzc || !fft_lb) return CHAPSIM_ERR_ARG;
-  *rhs_nzc = ctx->rhs_nzc;
+  *rhs_nzc = rhs_march(ctx);
   *fft_lb = ctx->fft_lb;
   return CHAPSIM_OK;
 }

@@ -128,10 +128,11 @@ static int time_substeps(chapsim_ctx *c, int reps, float *ms) {
   return rc;
 }
 
-// Time every candidate launch shape of one channel and keep the fastest.
-// The fields the trial substeps overwrite are saved first; on every exit
-// after the save (success or a failed trial) they are copied back and the
-// save buffer is freed, so a failure never leaves trial state behind.
+// Time every candidate launch shape of one channel and keep the fastest (the
+// shapes it had, when a trial fails).  The fields the trial substeps overwrite
+// are saved first; on every exit after the save (success or a failed trial)
+// they are copied back and the save buffer is freed, so a failure never leaves
+// trial state behind.
 static int autotune_channel(chapsim_batch *b, chapsim_ctx *c, int reps) {
   const size_t n = (size_t)c->d.sz * c->d.nz;
   const size_t tsz = c->cfg.precision == CHAPSIM_MIXED ? sizeof(float) : sizeof(double);
@@ -163,15 +164,20 @@ static int autotune_channel(chapsim_batch *b, chapsim_ctx *c, int reps) {
     b->err = "autotune: saving the channel state failed";
     return CHAPSIM_ERR_CUDA;
   }
-  // candidate launch shapes: RHS z segment x transform rows per block,
-  // then, with those fixed, the y-line block width of the Poisson solve
-  const int nzc_c[] = {8, 16, 32, 64};
+  // candidate launch shapes: RHS z segment (the present one and four others,
+  // launched as they are) x transform rows per block, then, with those fixed,
+  // the y-line block width of the Poisson solve
+  const int nzc_had = c->rhs_nzc, lb_had = c->fft_lb, ys_had = c->ys_bx;
+  const bool set_had = c->nzc_set;
+  const int nzc_c[] = {chapsim::rhs_march(c), 8, 16, 32, 64};
   const int lb_c[] = {0, 4, 8, 16};
   const int ys_c[] = {64, 128, 256};
   float best = 1e30f;
-  int bn = c->rhs_nzc, bl = c->fft_lb, by = c->ys_bx;
-  for (int nzc : nzc_c) {
-    if (nzc > c->d.nz || rc) continue;
+  int bn = nzc_c[0], bl = c->fft_lb, by = c->ys_bx;
+  c->nzc_set = true;
+  for (size_t q = 0; q < sizeof(nzc_c) / sizeof(int); ++q) {
+    const int nzc = nzc_c[q];
+    if (rc || (q && (nzc > c->d.nz || nzc == nzc_c[0]))) continue;
     for (int lb : lb_c) {
       c->rhs_nzc = nzc;
       c->fft_lb = lb;
@@ -190,6 +196,12 @@ static int autotune_channel(chapsim_batch *b, chapsim_ctx *c, int reps) {
     if (ms < best) { best = ms; by = ys; }
   }
   c->ys_bx = by;
+  if (rc) {
+    c->rhs_nzc = nzc_had;
+    c->nzc_set = set_had;
+    c->fft_lb = lb_had;
+    c->ys_bx = ys_had;
+  }
   // single exit: restore the saved state, then free the buffer
   const bool restored = copy_all(false) && cudaStreamSynchronize(c->stream) == cudaSuccess;
   if (!restored) cudaGetLastError();

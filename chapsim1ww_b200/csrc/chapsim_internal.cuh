@@ -180,8 +180,8 @@ struct chapsim_ctx {
   bool allow_band = true;   // banded x/z inverses when narrow enough
   bool fft_big = false;     // FFT plans with radix 7 or 11
   bool refine = true;       // mixed form: one FP64-residual refinement sweep
-  int rhs_nzc = 16;   // z planes per block of k_rhs_tma (autotunable)
-  bool nzc_set = false;  // the caller or the autotuner chose rhs_nzc / io_nzc (else march_len shortens it)
+  int rhs_nzc = 16;   // z planes per block of the momentum right-hand sides (autotunable; rhs_march)
+  bool nzc_set = false;  // the caller or the autotuner chose rhs_nzc (else rhs_march may shorten it)
   bool batched = false;  // a channel of a batch: its kernels share the chip with the other channels'
   int nsm = 148;      // multiprocessors of the device
   int fft_lb = 0;     // rows per block of the x transforms (0: default)
@@ -230,7 +230,6 @@ struct chapsim_ctx {
   CUtensorMap si_maps[4];  // semi-implicit scheme: mu, DRHOI_STG 1-3
   bool use_tma_si = false;
   bool use_tma_io = false;
-  int io_nzc = 16;  // z planes per block of the TMA momentum RHS
   bool si_smem_set = false;  // semi-implicit solve kernels got their shared-memory limit
   // property evaluation of the energy substep: table splines or the learned
   // model (a copy of a trained engine's model in context-owned buffers)
@@ -258,6 +257,15 @@ namespace chapsim {
 inline int march_len(int64_t tiles, int n, int len, int least, int want) {
   while (len / 2 >= least && tiles * ((n + len - 1) / len) < want) len /= 2;
   return len;
+}
+// z planes per block of the marching momentum right-hand sides (32 x 8 tiles):
+// the choice of the caller or the autotuner as it is, else rhs_nzc, shorter
+// where that gives fewer blocks than multiprocessors.  The mixed form keeps
+// rhs_nzc, and with it the bits of the mass-flux sum: its FP32 Poisson solve
+// magnifies them.
+inline int rhs_march(const chapsim_ctx *c) {
+  if (c->nzc_set || c->cfg.precision == CHAPSIM_MIXED) return c->rhs_nzc;
+  return march_len((int64_t)((c->d.nx + 31) / 32) * ((c->d.ny + 7) / 8), c->d.nz, c->rhs_nzc, 4, c->nsm);
 }
 // Phase timer mark: event slot ph of the substep being recorded (timing on).
 inline void phase_mark(chapsim_ctx *c, int ph) {

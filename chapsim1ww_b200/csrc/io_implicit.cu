@@ -975,7 +975,7 @@ int io_mom_si(chapsim_ctx *c, int ns, int *npart) {
     maps.m[S_M] = c->io_maps[4];
     maps.m[S_MU] = c->si_maps[0];
     for (int q = 0; q < 3; ++q) maps.m[S_R + q] = c->si_maps[1 + q];
-    const int nzc = c->nzc_set ? c->io_nzc : march_len((int64_t)grid.x * grid.y, d.nz, c->io_nzc, 4, c->nsm);
+    const int nzc = rhs_march(c);
     const dim3 g2(grid.x, grid.y, (d.nz + nzc - 1) / nzc), blk(SI_BX, SI_BY, 3);
     if (io.thermal)
       k_io_rhs_si_tma<true><<<g2, blk, st_smem(true), c->stream>>>(maps, d, io, sp.gam, sp.roh, sp.alp, c->io_cur, nzc);

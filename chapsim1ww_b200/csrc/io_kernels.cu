@@ -1566,13 +1566,6 @@ int io_therm_props(chapsim_ctx *c, int mode) {
   return CHAPSIM_OK;
 }
 
-// z planes per block of k_io_rhs_tma: the caller's choice, or 16, shorter
-// where that gives fewer blocks than multiprocessors (not in the mixed form,
-// whose FP32 Poisson solve magnifies the last bits of the mass-flux sum)
-static int io_march(const chapsim_ctx *c, dim3 grid) {
-  return c->nzc_set || c->cfg.precision == CHAPSIM_MIXED ? c->io_nzc : march_len((int64_t)grid.x * grid.y, c->d.nz, c->io_nzc, 4, c->nsm);
-}
-
 int io_mom(chapsim_ctx *c, int ns, bool prep) {
   TGDev &d = c->d;
   IODev &io = c->io;
@@ -1619,7 +1612,7 @@ int io_mom(chapsim_ctx *c, int ns, bool prep) {
   if (c->use_tma_io) {
     IoMaps maps;
     memcpy(maps.m, c->io_maps, sizeof(maps.m));
-    const int nzc = io_march(c, grid);
+    const int nzc = rhs_march(c);
     dim3 g2(grid.x, grid.y, (d.nz + nzc - 1) / nzc);
     constexpr size_t sm = ItGeo<false>::SMEM;
     if (io.thermal)
@@ -2273,7 +2266,7 @@ int io_np_mom(chapsim_ctx *c, int ns, bool mass_parts) {
   if (c->use_tma_io) {
     IoMaps maps;
     memcpy(maps.m, c->io_maps, sizeof(maps.m));
-    const int nzc = io_march(c, grid);
+    const int nzc = rhs_march(c);
     const dim3 g2(grid.x, grid.y, (d.nz + nzc - 1) / nzc);
     constexpr size_t sm = ItGeo<true>::SMEM;
     if (io.thermal)

@@ -1952,11 +1952,7 @@ template <typename T> struct Prec {
     {
       dim3 grid((d.nx + RHS_BX - 1) / RHS_BX, (d.ny + RHS_BY - 1) / RHS_BY, d.nz);
       if (c->use_tma_rhs) {
-        // (the mixed form keeps its block order, and with it the bits of the
-        // mass-flux sum: its FP32 Poisson solve magnifies them)
-        const int nzc = c->nzc_set || sizeof(T) == 4
-                            ? c->rhs_nzc
-                            : march_len((int64_t)grid.x * grid.y, d.nz, c->rhs_nzc, 4, c->nsm);
+        const int nzc = rhs_march(c);
         grid.z = (d.nz + nzc - 1) / nzc;
         RhsMaps maps;
         memcpy(maps.m, c->rhs_maps, sizeof(maps.m));

@@ -287,7 +287,8 @@ int chapsim_phase_reset(chapsim_ctx *ctx);
  * (rhs_nzc; on an IO context the momentum RHS) and rows per block of the x
  * transforms (fft_lb, 0 = default).
  * Results do not depend on fft_lb; rhs_nzc changes only the block order of
- * the mass-flux sum (round-off level). */
+ * the mass-flux sum (round-off level).  A length that was set is launched as
+ * it is; get_tuning gives the length in use. */
 int chapsim_set_tuning(chapsim_ctx *ctx, int rhs_nzc, int fft_lb);
 int chapsim_get_tuning(const chapsim_ctx *ctx, int *rhs_nzc, int *fft_lb);
 /* Spectral y-lines per block of the Poisson y-solve (64, 128 = default, or

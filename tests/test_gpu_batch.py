@@ -70,3 +70,27 @@ def test_mixed_batch_divergence_gate():
     for ch in b.channels:
         assert ch.divgck_tg() <= 1e-8
         assert ch.nan_count() == 0
+
+
+def test_tuned_march_is_the_one_that_runs():
+    """The march length that get_tuning reports, before and after autotune, is
+    the one launched: a channel that is given it explicitly leaves the same
+    bits (the mass-flux sum follows the march)."""
+    _need_gpu()
+    from chapsim1ww_b200 import ChannelBatch, TGChannel
+    b = ChannelBatch(CFGS)
+    b.init_random(seed=3, amp=0.1, project=True)
+    for tune in (False, True):
+        if tune:
+            b.autotune(reps=3)
+        shapes = [c.get_tuning() for c in b.channels]
+        b.init_random(seed=3, amp=0.1, project=True)
+        b.step(3)
+        b.sync()
+        for i, c in enumerate(CFGS):
+            s = TGChannel(**c)
+            s.set_tuning(*shapes[i])
+            s.random_fl_fld_tg(3 + i, 0.1, project=True)
+            s.step(3)
+            for n in ("u", "v", "w", "p"):
+                assert np.array_equal(s.get_field(n), b.channels[i].get_field(n)), (tune, i, n, shapes[i])
