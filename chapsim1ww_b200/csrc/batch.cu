@@ -165,12 +165,13 @@ static int autotune_channel(chapsim_batch *b, chapsim_ctx *c, int reps) {
     return CHAPSIM_ERR_CUDA;
   }
   // candidate launch shapes: RHS z segment (the present one and four others,
-  // launched as they are) x transform rows per block, then, with those fixed,
-  // the y-line block width of the Poisson solve
+  // launched as they are) x transform rows per block (where a kernel reads
+  // them), then, with those fixed, the y-line block width of the Poisson solve
   const int nzc_had = c->rhs_nzc, lb_had = c->fft_lb, ys_had = c->ys_bx;
   const bool set_had = c->nzc_set;
   const int nzc_c[] = {chapsim::rhs_march(c), 8, 16, 32, 64};
-  const int lb_c[] = {0, 4, 8, 16};
+  std::vector<int> lb_c{lb_had};
+  if (chapsim::reads_fft_lb(c)) lb_c = {0, 4, 8, 16};
   const int ys_c[] = {64, 128, 256};
   float best = 1e30f;
   int bn = nzc_c[0], bl = c->fft_lb, by = c->ys_bx;

@@ -284,6 +284,7 @@ inline void drop_substep_graphs(chapsim_ctx *c) {
 int flush_phase_events(chapsim_ctx *c);
 int launch_substep(chapsim_ctx *c, int ns);
 int launch_divg(chapsim_ctx *c, int ns);
+bool reads_fft_lb(const chapsim_ctx *c);  // whether the x transforms read fft_lb (the staged forward one does)
 int launch_pois3d(chapsim_ctx *c);
 int xnp_pivots(chapsim_ctx *c);
 int xnp_q_setup(chapsim_ctx *c);  // shared-memory limits of the quarter-wave FFT kernels

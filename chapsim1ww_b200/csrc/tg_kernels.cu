@@ -1836,17 +1836,21 @@ template <typename T> struct Prec {
     return true;
   }
 
+  // Whether the forward x transform of modes 0 and 1 takes register-blocked
+  // lines.  Powers of two keep the staged kernel: its index arithmetic is shifts and
+  // its inputs arrive by bulk copies (256 points: 150 us at 256x192x256
+  // against 171; 1024: 1415 against 1452 at 1024x384x256), where other
+  // lengths spend their time on divisions (384: 247 against 203 us at
+  // 384x192x192; 210: 80 against 62 us at 210x99x154).
+  static bool fftx_reg(const chapsim_ctx *c, XReg &x) {
+    return sizeof(T) == 8 && (c->d.nx & (c->d.nx - 1)) != 0 && x_reg(c, x);
+  }
+
   // mode 0: divergence of q; 1: stored RHSLLPHI; 2: residual buffer
   static int fftx(chapsim_ctx *c, int ns, int mode) {
     TGDev &d = c->d;
     XReg x;
-    // Powers of two keep the staged kernel: its index arithmetic is shifts and
-    // its inputs arrive by bulk copies (256 points: 150 us at 256x192x256
-    // against 171; 1024: 1415 against 1452 at 1024x384x256), where other
-    // lengths spend their time on divisions (384: 247 against 203 us at
-    // 384x192x192; 210: 80 against 62 us at 210x99x154).
-    const bool pow2 = (d.nx & (d.nx - 1)) == 0;
-    if (sizeof(T) == 8 && mode != 2 && !pow2 && x_reg(c, x)) {
+    if (mode != 2 && fftx_reg(c, x)) {
       auto k = x.p.rmax > 8 ? k_fftx_reg<16> : k_fftx_reg<8>;
       k<<<x.grid, x.threads, x.smem, c->stream>>>(d, c->sp[ns], x.p, x.per, mode);
       LAUNCHED();
@@ -2059,6 +2063,11 @@ int init_kernels(chapsim_ctx *c) {
   for (int s2 = 0; s2 < 16; ++s2)
     if (c->fx.rad[s2] == 7 || c->fx.rad[s2] == 11 || c->fz.rad[s2] == 7 || c->fz.rad[s2] == 11) c->fft_big = true;
   return c->cfg.precision == CHAPSIM_MIXED ? Prec<float>::init(c) : Prec<double>::init(c);
+}
+
+bool reads_fft_lb(const chapsim_ctx *c) {
+  Prec<double>::XReg x;
+  return c->cfg.precision == CHAPSIM_MIXED || !Prec<double>::fftx_reg(c, x);
 }
 
 int launch_divg(chapsim_ctx *c, int ns) {

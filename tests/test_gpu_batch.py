@@ -94,3 +94,17 @@ def test_tuned_march_is_the_one_that_runs():
             s.step(3)
             for n in ("u", "v", "w", "p"):
                 assert np.array_equal(s.get_field(n), b.channels[i].get_field(n)), (tune, i, n, shapes[i])
+
+
+def test_autotune_leaves_the_row_count_that_nothing_reads():
+    """The FP64 x transforms at lengths that are not powers of two do not read
+    fft_lb: the autotuner has nothing to choose there and keeps what was set."""
+    _need_gpu()
+    from chapsim1ww_b200 import ChannelBatch
+    cfgs = [dict(nx=n, ny=16, nz=16, ren=2500.0) for n in (24, 40, 48, 60, 80, 96, 112, 150)]
+    b = ChannelBatch(cfgs)
+    b.init_random(seed=3, amp=0.1, project=True)
+    for c in b.channels:
+        c.set_tuning(16, 2)
+    b.autotune(reps=2)
+    assert [c.get_tuning()[1] for c in b.channels] == [2] * len(cfgs)
