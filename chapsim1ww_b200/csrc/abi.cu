@@ -124,43 +124,6 @@ int circulant_band(int n, double a, double b, double qq, const double *pp, const
 
 }  // namespace
 
-// One substep call.  A host's time loop makes the same calls every step, and
-// launching a substep's ten to fifteen kernels one by one costs it 2.5 us
-// each (on the smallest grids more than they run), so from the third call of
-// a kind on the launches are captured once and replayed as one graph.  The
-// first two calls, timed phases, the coupled section (its launches reach into
-// the TG context) and a stream that the caller is capturing launch directly.
-template <typename F> static int run_substep(chapsim_ctx *ctx, chapsim_ctx::SubGraph &g, F launch) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  CKC(cudaStreamIsCapturing(ctx->stream, &cap));
-  if (ctx->timing || ctx->xnp || cap != cudaStreamCaptureStatusNone || g.calls < 2) {
-    ++g.calls;
-    return launch();
-  }
-  const int par = ctx->io_cur;
-  if (!g.exec) {
-    cudaGraph_t graph = nullptr;
-    const int64_t before = ctx->launches;
-    CKC(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = launch();
-    cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
-    g.kernels = ctx->launches - before;
-    ctx->launches = before;
-    ctx->io_cur = par;  // captured, not run
-    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
-    if (graph) cudaGraphDestroy(graph);
-    if (rc) return rc;
-    if (e != cudaSuccess) {
-      g.exec = nullptr;
-      ctx->err = cudaGetErrorString(e);
-      return CHAPSIM_ERR_CUDA;
-    }
-  }
-  CKC(cudaGraphLaunch(g.exec, ctx->stream));
-  ctx->launches += g.kernels;
-  return CHAPSIM_OK;
-}
-
 extern "C" {
 
 int chapsim_config_default(chapsim_config *cfg) {
@@ -187,7 +150,7 @@ int chapsim_config_default(chapsim_config *cfg) {
 // changes; a TG context's change also stales the pair graphs of the coupled
 // sections it feeds (they hold its kernels).
 static void drop_graphs(chapsim_ctx *ctx) {
-  chapsim::drop_substep_graphs(ctx);
+  ctx->sub.drop();
   if (ctx->step_graph) { cudaGraphExecDestroy(ctx->step_graph); ctx->step_graph = nullptr; }
   for (auto &g : ctx->io_graph)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
@@ -1171,7 +1134,7 @@ int chapsim_rk3_mom_tg(chapsim_ctx *ctx, int ns) {
   REQUIRE(ctx->domain == CHAPSIM_ITG, CHAPSIM_ERR_STATE, "not a TG context");
   REQUIRE(ns >= 0 && ns <= 3, CHAPSIM_ERR_ARG, "NS must be in 0..3");
   CKC(cudaSetDevice(ctx->device));
-  return run_substep(ctx, ctx->sub_mom[ns][0], [&] { return launch_substep(ctx, ns); });
+  return run_substep(ctx, ctx->sub.mom[ns][0], [&] { return launch_substep(ctx, ns); });
 }
 
 int chapsim_step_tg(chapsim_ctx *ctx, int nsteps) {
@@ -1446,7 +1409,7 @@ int chapsim_rk3_eng_io(chapsim_ctx *ctx, int ns) {
   REQUIRE(ctx->io.thermal, CHAPSIM_ERR_STATE, "thermal is off on this IO context");
   REQUIRE(ctx->has_table, CHAPSIM_ERR_STATE, "no property table");
   CKC(cudaSetDevice(ctx->device));
-  return run_substep(ctx, ctx->sub_eng[ns][ctx->io_cur], [&] { return io_eng(ctx, ns); });
+  return run_substep(ctx, ctx->sub.eng[ns][ctx->io_cur], [&] { return io_eng(ctx, ns); });
 }
 
 int chapsim_rk3_mom_io(chapsim_ctx *ctx, int ns) {
@@ -1455,7 +1418,7 @@ int chapsim_rk3_mom_io(chapsim_ctx *ctx, int ns) {
   REQUIRE(ns >= 0 && ns <= 3, CHAPSIM_ERR_ARG, "NS must be in 0..3");
   CKC(cudaSetDevice(ctx->device));
   const int par = ctx->io_cur;
-  const int rc = run_substep(ctx, ctx->sub_mom[ns][par], [&] { return io_mom(ctx, ns, ns >= 1); });
+  const int rc = run_substep(ctx, ctx->sub.mom[ns][par], [&] { return io_mom(ctx, ns, ns >= 1); });
   if (!rc) ctx->io_cur = 1 - par;  // G* is the new G, also after a replay
   return rc;
 }

@@ -208,7 +208,7 @@ static int autotune_channel(chapsim_batch *b, chapsim_ctx *c, int reps) {
   if (!restored) cudaGetLastError();
   cudaFree(sp);
   if (c->step_graph) { cudaGraphExecDestroy(c->step_graph); c->step_graph = nullptr; }
-  chapsim::drop_substep_graphs(c);
+  c->sub.drop();
   if (rc) return rc;
   if (!restored) {
     b->err = "autotune: restoring the channel state failed";

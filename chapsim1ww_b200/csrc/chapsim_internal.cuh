@@ -11,6 +11,7 @@
 #include "../../include/chapsim.h"
 #include "mlp_tc.cuh"
 #include "spline.cuh"
+#include "substep_graph.cuh"
 
 namespace chapsim {
 
@@ -202,14 +203,7 @@ struct chapsim_ctx {
   // m < nx, and 1 / SCALX of the forward transform
   double2 *xnp_qw = nullptr;
   double xnp_rscal = 1.0;
-  // the captured launches of one substep call (chapsim_rk3_mom_tg / _mom_io /
-  // _eng_io), by NS and the IO's io_cur
-  struct SubGraph {
-    cudaGraphExec_t exec = nullptr;
-    int64_t kernels = 0;
-    int calls = 0;
-  };
-  SubGraph sub_mom[4][2], sub_eng[4][2];
+  chapsim::SubGraphs sub;  // captured substep calls
   // CUDA graph of one full step (NS = 1, 2, 3)
   cudaGraphExec_t step_graph = nullptr;
   int64_t kernels_per_step = 0;
@@ -272,15 +266,6 @@ inline void phase_mark(chapsim_ctx *c, int ph) {
   if (c->timing) cudaEventRecord(c->evpool[(size_t)c->ev_pending * (CHAPSIM_PH_COUNT + 1) + ph], c->stream);
 }
 int init_kernels(chapsim_ctx *c);
-// captured substep calls go stale when a launch shape or a table changes
-inline void drop_substep_graphs(chapsim_ctx *c) {
-  for (auto *set : {c->sub_mom, c->sub_eng})
-    for (int ns = 0; ns < 4; ++ns)
-      for (int par = 0; par < 2; ++par) {
-        if (set[ns][par].exec) cudaGraphExecDestroy(set[ns][par].exec);
-        set[ns][par] = chapsim_ctx::SubGraph();
-      }
-}
 int flush_phase_events(chapsim_ctx *c);
 int launch_substep(chapsim_ctx *c, int ns);
 int launch_divg(chapsim_ctx *c, int ns);
