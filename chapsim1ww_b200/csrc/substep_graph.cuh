@@ -5,8 +5,6 @@
 #include <cuda_runtime_api.h>
 #include <stdint.h>
 
-#include "../../include/chapsim.h"
-
 namespace chapsim {
 
 // The captured launches of one kind of substep call.
@@ -14,6 +12,7 @@ struct SubGraph {
   cudaGraphExec_t exec = nullptr;
   int64_t kernels = 0;
   int calls = 0, replays = 0;
+  bool off = false;  // capturing failed: launched directly
 };
 
 // A context's captures by NS and the IO's io_cur, and the calls of a kind that
@@ -52,41 +51,45 @@ struct SubGraphs {
 // each (on the smallest grids more than they run), so after the first calls of
 // a kind the launches are captured once and replayed as one graph.  Those
 // first calls, timed phases, the coupled section (its launches reach into the
-// TG context) and a stream that the caller is capturing launch directly.
+// TG context) and a stream that the caller is capturing launch directly, and
+// so does a kind whose capture fails (a graph takes device memory that a
+// launch does not).
 template <typename Ctx, typename F> int run_substep(Ctx *ctx, SubGraph &g, F launch) {
-  auto failed = [&](cudaError_t e) {
-    ctx->err = cudaGetErrorString(e);
-    return CHAPSIM_ERR_CUDA;
-  };
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(ctx->stream, &cap);
-  if (e != cudaSuccess) return failed(e);
-  if (ctx->timing || ctx->xnp || cap != cudaStreamCaptureStatusNone || g.calls < ctx->sub.wait) {
+  if (g.off || ctx->timing || ctx->xnp || g.calls < ctx->sub.wait ||
+      cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
     ++g.calls;
     return launch();
   }
   const int par = ctx->io_cur;
+  cudaError_t e = cudaSuccess;
   if (!g.exec) {
     cudaGraph_t graph = nullptr;
     const int64_t before = ctx->launches;
-    if ((e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return failed(e);
-    const int rc = launch();
-    e = cudaStreamEndCapture(ctx->stream, &graph);
+    int rc = 0;
+    e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      rc = launch();
+      e = cudaStreamEndCapture(ctx->stream, &graph);
+    }
     g.kernels = ctx->launches - before;
     ctx->launches = before;
     ctx->io_cur = par;  // captured, not run
-    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
+    if (e == cudaSuccess) e = rc ? cudaErrorUnknown : cudaGraphInstantiate(&g.exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
-    if (rc) return rc;
-    if (e != cudaSuccess) {
-      g.exec = nullptr;
-      return failed(e);
-    }
+    if (e != cudaSuccess) g.exec = nullptr;
   }
-  if ((e = cudaGraphLaunch(g.exec, ctx->stream)) != cudaSuccess) return failed(e);
+  if (g.exec) e = cudaGraphLaunch(g.exec, ctx->stream);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+    g.off = true;
+    return launch();
+  }
   ++g.replays;
   ctx->launches += g.kernels;
-  return CHAPSIM_OK;
+  return 0;
 }
 
 }  // namespace chapsim

@@ -103,6 +103,16 @@ int main(int argc, char **argv) {
     c.xnp = 1;
     for (int s = 0; s < 10; ++s) CHECK(c.step() == 0);
     CHECK(captures == 0 && c.direct == 90 && c.launches == 270);
+  } else if (what == "fails") {  // no memory for a graph: the calls go on, and capture again after a drop
+    int &f = argv[2] == std::string("begin") ? fail_begin : argv[2] == std::string("instantiate") ? fail_inst : fail_launch;
+    f = 1;
+    for (int s = 0; s < 10; ++s) CHECK(c.step() == 0);
+    CHECK(c.direct == 30 && c.launches == 90 && c.io_cur == 0 && graph_launches == 0 && live == 0);
+    CHECK(begins <= 6);  // one try a kind
+    f = 0;
+    c.sub.drop();
+    for (int s = 0; s < 10; ++s) CHECK(c.step() == 0);
+    CHECK(c.direct == 30 + 12 && graph_launches == 30 - 12 && c.launches == 180);
   }
   return 0;
 }
@@ -140,3 +150,8 @@ def test_captures_that_do_not_pay_are_given_up(prog, period, most):
 
 def test_calls_that_launch_directly(prog):
     run(prog, "direct")
+
+
+@pytest.mark.parametrize("call", ["begin", "instantiate", "launch"])
+def test_failed_captures_launch_directly(prog, call):
+    run(prog, "fails", call)
