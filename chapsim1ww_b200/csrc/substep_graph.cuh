@@ -67,6 +67,11 @@ template <typename Ctx, typename F> int run_substep(Ctx *ctx, SubGraph &g, F lau
     cudaGraph_t graph = nullptr;
     const int64_t before = ctx->launches;
     int rc = 0;
+    // The caller's thread, or another one in the global mode, may be capturing
+    // a stream of its own, and cudaGraphInstantiate is a call that would end
+    // that capture: this one has nothing to do with it.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
       rc = launch();
@@ -77,6 +82,7 @@ template <typename Ctx, typename F> int run_substep(Ctx *ctx, SubGraph &g, F lau
     ctx->io_cur = par;  // captured, not run
     if (e == cudaSuccess) e = rc ? cudaErrorUnknown : cudaGraphInstantiate(&g.exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     if (e != cudaSuccess) g.exec = nullptr;
   }
   if (g.exec) e = cudaGraphLaunch(g.exec, ctx->stream);

@@ -359,3 +359,31 @@ def test_adi_first_plane_of_a_march(dt, ren):
             assert (err <= TOL).all(), (ns, np.flatnonzero(err > TOL), err.max())
         runs.append(v)
     assert np.array_equal(*runs)
+
+
+@pytest.mark.parametrize("mode", ["relaxed", "thread_local", "global"])
+def test_substep_calls_beside_a_capture_of_the_caller(mode):
+    """Substep calls, those that are captured among them, while the caller
+    captures a stream of its own: neither disturbs the other."""
+    _need_gpu()
+    import torch
+    from chapsim1ww_b200 import TGChannel
+    g, ref = TGChannel(32, 24, 16), TGChannel(32, 24, 16)
+    for x in (g, ref):
+        x.random_fl_fld_tg(1, 0.1)
+    ref.step(6)
+    ref.sync()
+    a, b = torch.ones(64, device="cuda"), torch.zeros(64, device="cuda")
+    torch.cuda.synchronize()
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode=mode):
+        b.add_(a)
+        for _ in range(6):
+            for ns in (1, 2, 3):
+                g.solverrk3_mom_tg(ns)
+        b.add_(a)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert b.eq(2.0).all()
+    for n in ("u", "v", "w", "p"):
+        assert np.array_equal(g.get_field(n), ref.get_field(n)), n

@@ -47,6 +47,13 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) {
   ++graph_launches;
   return cudaSuccess;
 }
+static cudaStreamCaptureMode thread_mode = cudaStreamCaptureModeGlobal;
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *m) {
+  const cudaStreamCaptureMode was = thread_mode;
+  thread_mode = *m;
+  *m = was;
+  return cudaSuccess;
+}
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "fake"; }
 }
@@ -114,6 +121,7 @@ int main(int argc, char **argv) {
     for (int s = 0; s < 10; ++s) CHECK(c.step() == 0);
     CHECK(c.direct == 30 + 12 && graph_launches == 30 - 12 && c.launches == 180);
   }
+  CHECK(thread_mode == cudaStreamCaptureModeGlobal);
   return 0;
 }
 """
