@@ -121,6 +121,7 @@ struct Grp {
 };
 template <class S>
 __device__ __forceinline__ Grp grp_of(const S &s) {
+  if constexpr (S::G == 1) return {(int)threadIdx.x, 0, s.tmem};  // a group index known to be 0
   const int g = threadIdx.x / TILE;
   return {(int)threadIdx.x % TILE, g, s.tmem + (uint32_t)(TMEM_COLS * g)};
 }
@@ -470,11 +471,18 @@ template <class S>
 __device__ __forceinline__ bool tile_eval(S &s, const Grp &q, float x, float (&y)[NO], uint32_t &phase, int *err) {
   uint16_t *a_hi = s.ops[q.g][0], *a_lo = s.ops[q.g][1];
   const uint32_t lane_base = q.tm + ((uint32_t)(q.r & ~31) << 16);
-  float a[32];
+  // halves of the hidden units in registers at a time: both with the 128
+  // registers of four one-group CTAs per SM, one beside the energy substep's
+  // own values (THERM_PROP_UPDATE at 384x192x192: 1055 us, 1083 with one at a
+  // time; 1043 with the group index of a one-group CTA known, grp_of)
+  constexpr int HP = S::G == 1 ? 2 : 1;
+  float a[32 * HP];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    layer1_32(s.w1 + 32 * h, s.b1 + 32 * h, x, a);
-    store_split32(a_hi, a_lo, q.r, 32 * h, a);
+  for (int h0 = 0; h0 < 2; h0 += HP) {
+#pragma unroll
+    for (int h = 0; h < HP; ++h) layer1_32(s.w1 + 32 * (h0 + h), s.b1 + 32 * (h0 + h), x, a + 32 * h);
+#pragma unroll
+    for (int h = 0; h < HP; ++h) store_split32(a_hi, a_lo, q.r, 32 * (h0 + h), a + 32 * h);
   }
   chapsim::fence_proxy_async();
   tc_fence_before();
@@ -486,10 +494,15 @@ __device__ __forceinline__ bool tile_eval(S &s, const Grp &q, float x, float (&y
   }
   if (!layer_wait(s, q, phase, err)) return false;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {  // the layer-2 MMAs have completed: the A tiles are free
-    tmem_ld32(lane_base + 32 * h, a);
-    bias_tanh32(s.b2 + 32 * h, a);
-    store_split32(a_hi, a_lo, q.r, 32 * h, a);
+  for (int h0 = 0; h0 < 2; h0 += HP) {  // the layer-2 MMAs have completed: the A tiles are free
+    if constexpr (HP == 2)
+      tmem_ld32x2(lane_base, lane_base + 32, a, a + 32);
+    else
+      tmem_ld32(lane_base + 32 * h0, a);
+#pragma unroll
+    for (int h = 0; h < HP; ++h) bias_tanh32(s.b2 + 32 * (h0 + h), a + 32 * h);
+#pragma unroll
+    for (int h = 0; h < HP; ++h) store_split32(a_hi, a_lo, q.r, 32 * (h0 + h), a + 32 * h);
   }
   chapsim::fence_proxy_async();
   tc_fence_before();
