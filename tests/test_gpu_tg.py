@@ -387,3 +387,25 @@ def test_substep_calls_beside_a_capture_of_the_caller(mode):
     assert b.eq(2.0).all()
     for n in ("u", "v", "w", "p"):
         assert np.array_equal(g.get_field(n), ref.get_field(n)), n
+
+
+@pytest.mark.parametrize("nx", [28, 44, 54, 60, 66, 70, 84, 90, 98, 126, 144, 150, 162, 176, 210, 216, 242, 264, 288, 300, 324, 330, 350,
+                                360, 384, 432, 450, 462, 486, 588, 630])
+def test_x_transform_lengths_on_more_lines(nx):
+    """The x transforms over their radices on enough lines for the register-
+    blocked forward form, with an odd row count; the short list of
+    test_x_transform_lengths takes the staged one at most lengths."""
+    g, o = pair(nx, 11, 240, seed=4)
+    g.solverrk3_mom_tg(0)
+    o.substep(0)
+    compare(g, o, tag=f"nx {nx}")
+
+
+@pytest.mark.parametrize("dims", [(1250, 5, 8), (1458, 6, 8), (10, 5, 750), (10, 6, 924), (16, 9, 1008)])
+def test_transform_lengths_without_a_register_plan(dims):
+    """FP64 lengths that the staged kernels serve: x without a plan of three
+    radices up to 16 (both directions), z with too many threads a line."""
+    g, o = pair(*dims, seed=4)
+    g.solverrk3_mom_tg(0)
+    o.substep(0)
+    compare(g, o, tag=str(dims))
