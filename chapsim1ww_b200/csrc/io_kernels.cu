@@ -132,11 +132,11 @@ struct Look {
 // ---------------------------------------------------------------- energy
 // RHS_ENERGY_EXPLICIT and the RHOH update of SOLVERRK3_ENG_IO (:22-35):
 // rhoh += gam dt R + zeta dt R_old, limited to RHOHmax + REALMIN.  This form,
-// one cell per thread, serves grids too small for the TMA boxes and the mixed
-// form (whose FP32 Poisson solve magnifies a change of the last bits); the
-// others take k_io_eng_rhs_tma.  Six blocks
-// per SM (40 registers): latency-bound on its neighbour loads, it gains from
-// the extra resident warps (measured 0.536 -> 0.510 ms at 512x192x256).
+// one cell per thread, serves grids too small for the TMA boxes or for marches
+// (eng_march) and the mixed form (whose FP32 Poisson solve magnifies a change of
+// the last bits); the others take k_io_eng_rhs_tma.  Six blocks per SM (40
+// registers): latency-bound on its neighbour loads, it gains from the extra
+// resident warps (measured 0.536 -> 0.510 ms at 512x192x256).
 __global__ void __launch_bounds__(IO_BX *IO_BY, 6) k_io_eng_rhs(TGDev d, IODev io, double cdt1, double cdt0, int cur) {
   const int nx = d.nx, ny = d.ny;
   const int i = blockIdx.x * IO_BX + threadIdx.x;
@@ -866,10 +866,10 @@ static_assert((ItGeo<true>::PST * 8) % 128 == 0 && ItGeo<true>::PST >= ItGeo<tru
 // neighbours, plane k + 1 for the column ahead, plane k + 2 in flight; the
 // plane behind and the z fluxes stay in registers.  62 KB let three blocks
 // share a multiprocessor.  The kernel of one cell per thread issues 37 loads
-// and waits for them (DRAM 48 %): 0.351 -> 0.275 ms at 384x192x192, 0.615 ->
-// 0.446 at 512x192x256 coupled, 16.5 -> 15.7 us at 100x49x60; its bytes take
-// 0.228 ms at 384x192x192.  16 planes a block: 0.275 at 8, 0.279 at 32, 0.308
-// at 64 (the planes of many long marches fall out of L2 between tiles).
+// and waits for them (DRAM 48 %): 0.348 -> 0.272 ms at 384x192x192, 0.615 ->
+// 0.446 at 512x192x256 coupled; its bytes take 0.228 ms at 384x192x192.  16
+// planes a block: 0.275 at 8, 0.280 at 32 (the planes of many long marches fall
+// out of L2 between tiles); which grids march, and how far: eng_march.
 constexpr int ET_NF = 7, E_H = 0, E_T = 1, E_K = 2, E_GX = 3, E_HX = 4, E_GY = 5, E_HY = 6;
 template <bool CPL> constexpr size_t et_smem() {
   return (size_t)3 * ET_NF * ItGeo<CPL>::PST * sizeof(double) + 3 * sizeof(uint64_t);
@@ -1514,12 +1514,28 @@ int io_np_mom(chapsim_ctx *c, int ns, bool mass_parts);
 // Phase-timer slots of an IO substep, in execution order: 0 energy RHS,
 // 1 property update + wall ghosts, 2 prep (DrhoDtP, u = G / rho), 3 momentum
 // RHS + DPGRNS, 4-8 the Poisson transforms and y-solve, 9 correction.
+// z planes per block of k_io_eng_rhs_tma, 0: one cell per thread.  A march
+// starts with two planes that nothing hides, so it wants four blocks of four
+// planes a multiprocessor, or nearly a full wave of three; it grows to 8 and 16
+// planes where that leaves 13 blocks each.  Cell / march of 4 / 8 / 16 in us:
+// 8.9 / 12.7 / 14.4 / 22.6 at 40x54x44 (154 blocks of 4), 17.5 / 19.3 / 20.4 /
+// 27.7 at 128x64x64 (512), 14.3 / 13.3 / 17.4 / 25.4 at 100x49x60 (420), 26.6 /
+// 24.6 / 24.5 / 34.9 at 160x96x50 (780), 50 / 46 / 49 / 60 at 66x33x500 (1875).
+// Over 150 drawn grids 0.92 of the cell kernel's time, within 1 % of the best.
+static int eng_march(const chapsim_ctx *c, dim3 grid) {
+  if (!c->use_tma_io || c->cfg.precision == CHAPSIM_MIXED) return 0;
+  const int64_t tiles = (int64_t)grid.x * grid.y, b4 = tiles * ((c->d.nz + 3) / 4);
+  if (b4 < 4 * c->nsm && (b4 > 3 * c->nsm || 4 * b4 < 11 * c->nsm)) return 0;
+  return march_len(tiles, c->d.nz, 16, 4, c->nsm * 27 / 2);
+}
+
 int io_eng(chapsim_ctx *c, int ns) {
   TGDev &d = c->d;
   const SubParams &sp = c->sp[ns];
   phase_mark(c, 0);
   const dim3 grid = cell_grid(d), blk(IO_BX, IO_BY);
-  if (c->use_tma_io && c->cfg.precision != CHAPSIM_MIXED) {
+  const int nzc = eng_march(c, grid);
+  if (nzc) {
     EngMaps maps;
     const int cur = c->io_cur;
     memcpy(maps.m, c->eng_maps, sizeof(c->eng_maps));
@@ -1527,7 +1543,6 @@ int io_eng(chapsim_ctx *c, int ns) {
       maps.m[E_GX + 2 * q] = c->io_maps[5 + 3 * cur + q];
       maps.m[E_HX + 2 * q] = c->io_maps[5 + 3 * (1 - cur) + q];
     }
-    const int nzc = march_len((int64_t)grid.x * grid.y, d.nz, 16, 4, 2 * c->nsm);
     const dim3 g3(grid.x, grid.y, (d.nz + nzc - 1) / nzc);
     if (c->xnp)
       k_io_eng_rhs_tma<true><<<g3, blk, et_smem<true>(), c->stream>>>(maps, d, c->io, sp.gam * d.dt, sp.roh * d.dt,

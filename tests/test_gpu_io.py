@@ -353,3 +353,23 @@ def test_energy_rhs_march_edges(dims):
         g.solverrk3_eng_io(ns)
         o.eng(ns)
         compare(g, o, THERMAL, tag=f"eng{ns}")
+
+
+@pytest.mark.parametrize("dims", [(36, 9, 600), (50, 20, 500), (66, 17, 270), (98, 33, 126), (100, 49, 60), (160, 130, 280), (256, 65, 500)],
+                         ids=lambda d: "x".join(map(str, d)))
+def test_energy_rhs_march_lengths(dims):
+    """The energy substep on grids with enough tiles to march: 4, 8 and 16
+    planes a block, short last marches and partial tiles (the smaller grids of
+    test_energy_rhs_march_edges take one cell per thread)."""
+    g, o = pair(*dims, thermal=1)
+    rng = np.random.default_rng(12)
+    rhoh = 0.3 * rng.uniform(-1.0, 1.0, g.shape)
+    T = 1.0 + 0.2 * rng.uniform(-1.0, 1.0, g.shape)
+    for x, put in ((g, g.set_field), (o, o.set)):
+        put("h", rhoh)
+        put("t", T)
+        put("rhoh", rhoh)
+    for ns in (1, 2):
+        g.solverrk3_eng_io(ns)
+        o.eng(ns)
+        compare(g, o, THERMAL, tag=f"eng{ns}")
