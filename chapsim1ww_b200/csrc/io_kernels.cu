@@ -205,7 +205,10 @@ __global__ void __launch_bounds__(IO_BX *IO_BY, 6) k_io_eng_rhs(TGDev d, IODev i
 // 384x192x192 with enthalpies varying from cell to cell, against 0.19 ms for
 // its bytes, since the look-ups read pair arrays instead of interval records
 // and the second look-up reuses the first one's interval.  Five blocks per
-// SM: 0.421 ms at four (56 registers), 0.399 ms at six (spills).
+// SM: 0.421 ms at four (56 registers), 0.399 ms at six (spills).  Where the
+// enthalpy hardly varies the wait for the loads bounds it: rho h is loaded with
+// rho and mu, not after their stores (0.289 -> 0.247 ms at 384x192x192 with one
+// enthalpy, 0.249 with records; 0.347 -> 0.324 with a smooth field).
 __global__ void __launch_bounds__(IO_BX *IO_BY, 5) k_io_eng_props(TGDev d, IODev io) {
   const int nx = d.nx, ny = d.ny;
   const int i = blockIdx.x * IO_BX + threadIdx.x;
@@ -213,14 +216,14 @@ __global__ void __launch_bounds__(IO_BX *IO_BY, 5) k_io_eng_props(TGDev d, IODev
   const int k = blockIdx.z;
   if (i >= nx || j > ny + 1) return;
   const int64_t c = i + d.sy * j + d.sz * k;
-  const double dold = io.D[c], muold = io.mu[c];
+  const bool wall = j < 1 || j > ny;
+  const double dold = io.D[c], muold = io.mu[c], rh = wall ? 0.0 : io.rhoh[c];
   io.mu0[c] = muold;
   io.D0[c] = dold;
-  if (j < 1 || j > ny) {
+  if (wall) {
     io.msum[c] = muold + muold;  // ghost rows: the ghost kernel sets the new value
     return;
   }
-  const double rh = io.rhoh[c];
   int bad = 0;
   double h = rh / dold, T, D = dold;
   Look look;
