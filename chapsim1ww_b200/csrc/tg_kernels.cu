@@ -1901,16 +1901,23 @@ template <typename T> struct Prec {
   // The z transforms of the spectral descriptor s, sign -1 forward: register-
   // blocked in FP64 where the plan's blocks hold two lines or more, else (and
   // for FP32 spectra, whose roundings the refined solve magnifies) in shared
-  // memory.
+  // memory.  Blocks of two lines (32 bytes of a row) against staged ones of
+  // four or more pay on grids of many blocks (both transforms, staged / register
+  // in us: 175 / 158 at 192x130x360, 223 / 157 at 420) and lose a little on few
+  // (48x40 in x and y: 32 / 34 at 360, 33 / 39 at 480, 37 / 41 at 576), except
+  // where the staged form takes five stages or has a factor 11 (41 / 39 at 486).
   static int fftz(chapsim_ctx *c, const TGDev &s, int sign) {
     RegPlan p = c->rz;
     p.tw = c->fz.tw64;
     int llz = 3;
     const int per = reg_per(p);
     while (llz > 0 && (per << llz) > 256) --llz;
-    if (sizeof(T) == 8 && p.nst && llz >= 1) {
+    const dim3 rgrid((s.lh + (1 << llz) - 1) >> llz, s.ny);
+    const bool few = llz == 1 && fftz_lz(s.nz) >= 4 && c->fz.nrad <= 4 && s.nz % 11 != 0 &&
+                     (int64_t)rgrid.x * rgrid.y < 8 * c->nsm;
+    if (sizeof(T) == 8 && p.nst && llz >= 1 && !few) {
       const int lz = 1 << llz;
-      const dim3 grid((s.lh + lz - 1) / lz, s.ny);
+      const dim3 grid = rgrid;
       const size_t sm = (size_t)lz * p.n * sizeof(double2);
       auto k = p.rmax > 8 ? (sign < 0 ? k_fftz_reg<16, -1> : k_fftz_reg<16, 1>)
                           : (sign < 0 ? k_fftz_reg<8, -1> : k_fftz_reg<8, 1>);

@@ -409,3 +409,13 @@ def test_transform_lengths_without_a_register_plan(dims):
     g.solverrk3_mom_tg(0)
     o.substep(0)
     compare(g, o, tag=str(dims))
+
+
+@pytest.mark.parametrize("dims", [(10, 5, 360), (10, 5, 504), (66, 100, 360), (66, 100, 504)])
+def test_z_transform_forms_by_grid(dims):
+    """z lengths whose register lines come two to a block: staged on few
+    blocks, register-blocked on many."""
+    g, o = pair(*dims, seed=4)
+    g.solverrk3_mom_tg(0)
+    o.substep(0)
+    compare(g, o, tag=str(dims))
