@@ -790,9 +790,7 @@ static bool launch_adixz_rows(cudaStream_t st, const TGDev &d, const SubParams &
 // before; with the next tile in registers 0.219 ms).
 constexpr int AY_JT = 32, AY_TX = 32, AY_TY = 8, AYB_WMAX = 16, AY_R = AY_JT / AY_TY;
 constexpr int AY_TW[6] = {2, 4, 6, 8, 12, 16};  // compiled widths
-// planes per block, at most: 256x192x256 192 us (194 at 16), 210x99x154 71 (73),
-// 66x33x500 45 (52); shorter ones take 210 and 75 us at 4
-constexpr int AY_SEG = 8;
+constexpr int AY_SEG = 16;                      // planes per block, at most
 constexpr int AY_PD = 4;                        // tiles of the ring
 static_assert(AY_TW[5] == AYB_WMAX, "the widest compiled band is the host's limit");
 template <typename T, int W>
@@ -934,9 +932,15 @@ static void launch_adiy(const chapsim_ctx *c, const TGDev &d, const SubParams &s
   int q = 0;
   while (q < 5 && sp.wy > AY_TW[q]) ++q;
   dim3 grid((d.nx + AY_TX - 1) / AY_TX, (d.ny + AY_JT - 1) / AY_JT, 1);
-  // shorter marches below 2.4 blocks per SM (100x49x60: 360 blocks of 4 planes
-  // 15.2 us, 720 of 2 16.6; 360x40x48: 432 of 8 23.4, 864 of 4 24.9)
-  const int seg = march_len((int64_t)3 * grid.x * grid.y, d.nz, AY_SEG, 2, c->nsm * 12 / 5);
+  // Full marches where they give four and a half blocks per SM (256x192x256,
+  // 2304 blocks: a step among others takes 0.7 % less than with 8 planes),
+  // else half of it (66x33x500: 45 us, 576 blocks of 16 planes 52), shorter ones
+  // below 2.4 blocks per SM (100x49x60: 360 blocks of 4 planes 15.2 us, 720 of 2
+  // 16.6; 360x40x48: 432 of 8 23.4, 864 of 4 24.9).
+  const int64_t tiles = (int64_t)3 * grid.x * grid.y;
+  const int seg = 2 * tiles * ((d.nz + AY_SEG - 1) / AY_SEG) >= 9 * c->nsm
+                      ? AY_SEG
+                      : march_len(tiles, d.nz, AY_SEG / 2, 2, c->nsm * 12 / 5);
   grid.z = 3 * ((d.nz + seg - 1) / seg);
   fns[q](grid, c->stream, d, sp, seg);
 }
