@@ -1518,18 +1518,21 @@ int io_np_mom(chapsim_ctx *c, int ns, bool mass_parts);
 // 1 property update + wall ghosts, 2 prep (DrhoDtP, u = G / rho), 3 momentum
 // RHS + DPGRNS, 4-8 the Poisson transforms and y-solve, 9 correction.
 // z planes per block of k_io_eng_rhs_tma, 0: one cell per thread.  A march
-// starts with two planes that nothing hides, so it wants four blocks of four
-// planes a multiprocessor, or nearly a full wave of three; it grows to 8 and 16
-// planes where that leaves 13 blocks each.  Cell / march of 4 / 8 / 16 in us:
-// 8.9 / 12.7 / 14.4 / 22.6 at 40x54x44 (154 blocks of 4), 17.5 / 19.3 / 20.4 /
-// 27.7 at 128x64x64 (512), 14.3 / 13.3 / 17.4 / 25.4 at 100x49x60 (420), 26.6 /
-// 24.6 / 24.5 / 34.9 at 160x96x50 (780), 50 / 46 / 49 / 60 at 66x33x500 (1875).
-// Over 150 drawn grids 0.92 of the cell kernel's time, within 1 % of the best.
+// starts with two planes that nothing hides, and many long ones leave the last
+// multiprocessors alone; but it loads less, so that where other contexts fill
+// the gaps longer ones are better.  The line lies where neither use loses
+// much.  Whole energy substep, one context waited for / three taking turns, in
+// us, one cell - 4 - 8 - 16 planes:
+//   84x33x50 (195 blocks of 4)     17 - 21 - 23 - 33 /  7.7 -  8.5 -  9.9 - 12.3
+//   192x55x44 (462)                29 - 29 - 29 - 37 / 25.0 - 23.2 - 23.0 - 25.6
+//   160x96x50 (780)                45 - 45 - 43 - 55 / 38.1 - 36.4 - 35.5 - 34.1
+//   192x77x176 (2640)         128 - 119 - 119 - 126 / 114.8 - 108.4 - 106.8 - 104.8
+//   384x192x192 (13824)       622 - 552 - 554 - 554 / 612.2 - 573.3 - 559.7 - 551.6
 static int eng_march(const chapsim_ctx *c, dim3 grid) {
   if (!c->use_tma_io || c->cfg.precision == CHAPSIM_MIXED) return 0;
-  const int64_t tiles = (int64_t)grid.x * grid.y, b4 = tiles * ((c->d.nz + 3) / 4);
-  if (b4 < 4 * c->nsm && (b4 > 3 * c->nsm || 4 * b4 < 11 * c->nsm)) return 0;
-  return march_len(tiles, c->d.nz, 16, 4, c->nsm * 27 / 2);
+  const int64_t blocks4 = (int64_t)grid.x * grid.y * ((c->d.nz + 3) / 4);
+  if (2 * blocks4 < 3 * c->nsm) return 0;
+  return blocks4 < 4 * c->nsm ? 4 : (blocks4 < 40 * c->nsm ? 8 : 16);
 }
 
 int io_eng(chapsim_ctx *c, int ns) {

@@ -1850,36 +1850,30 @@ template <typename T> struct Prec {
   // Whether the forward x transform of modes 0 and 1 takes register-blocked
   // lines.  The staged kernel copies its rows ahead but divides per butterfly
   // at lengths that are not powers of two and crosses shared memory once per
-  // radix; the register lines load straight from global memory and wait for
-  // it.  Measured staged / register, in us, over 130 lengths of TG and IO grids
-  // of 8.0, 1.2 and 0.25 M cells (the rule's mean over both is within 1 % of
-  // the better one each time; 3 % where all lengths but powers of two take
-  // registers, at most 19 % against 35 %):
-  //  - lengths up to 22: 41 / 25 at 10, 49 / 48 at 24;
+  // radix; the register lines load straight from global memory, which pays
+  // while u, v and w come out of the L2 (DIVG alone at 0.4 and 2 M cells, 100
+  // lengths: 0.8 and 0.7 of the staged time).  Powers of two are staged: 97 /
+  // 117 us (staged / register) at 128, 102 / 117 at 256, 128 / 139 at 1024 for 8 M
+  // cells, 22 / 22, 22 / 23 and 25 / 23 for 1.2 M; 78 / 110 and 21 / 23 at 64.
+  // Where the inputs come from DRAM (8 M cells, in us) the register lines keep
   //  - factors 7 and 11, whose staged kernel has two blocks per SM: 176 / 129 at
   //    210, 181 / 150 at 352;
-  //  - where the staged rows of a multiprocessor are four or fewer: 172 / 160 at
-  //    900, 156 / 145 at 1152 (800, six rows: 125 / 151), and where it holds one
-  //    block: 228 / 148 at 1440;
-  //  - three radices up to 8 where u, v and w come out of the L2 (1.2 M cells:
-  //    29 / 22 at 54, 28 / 23 at 216), or, with DrhoDtP staged too, three lines
-  //    or fewer to a staged block (8 M cells, IO: 129 / 115 at 288, 146 / 104 at
-  //    384; TG: 127 / 134 and 123 / 124; 102 / 125 at 96);
-  //  - larger radices (two blocks of 128 registers per SM) only against five
-  //    staged stages or more: 186 / 156 at 486; 127 / 165 at 360, 125 / 152 at 640;
-  //  - too few lines or blocks for the chip wait for the staged kernel's fewer,
-  //    wider blocks: 12.3 / 16.3 at 448, 14.3 / 16.4 at 640, 14.6 / 18.6 at 132.
+  //  - lengths whose staged rows of a multiprocessor are four or fewer, 172 / 160
+  //    at 900 and 228 / 148 at 1440 (800, six rows: 125 / 151);
+  //  - with DrhoDtP staged too, radices up to 8 with three lines or fewer to a
+  //    staged block: 129 / 115 at 288, 146 / 104 at 384 (TG: 127 / 134, 123 / 124);
+  //  - five staged stages or more at two blocks per SM: 186 / 156 at 486;
+  // and are slower elsewhere: 102 / 125 at 96, 109 / 136 at 100, 106 / 126 at 160,
+  // 127 / 165 at 360, 125 / 152 at 640.
   static bool fftx_reg(const chapsim_ctx *c, XReg &x) {
     if (sizeof(T) != 8 || !x_reg(c, x)) return false;
     const int n = c->d.nx, lb = fftx_rows(c);
     const int per_sm = std::min(3, (int)(227 * 1024 / (fftx_smem(c, lb) + 1024)));  // staged blocks
-    if (n <= 22 || per_sm <= 1) return true;
-    const int64_t lines = (int64_t)((c->d.ny + 1) / 2) * c->d.nz, blocks = (int64_t)x.grid.x * x.grid.y;
-    if ((n & (n - 1)) == 0 || (lines < 2 * c->nsm && n % 11 != 0) || blocks < c->nsm * 3 / 4) return false;
+    if (n <= 22 || per_sm <= 1) return true;  // 41 / 25 us at 10, 41 / 32 at 16; 162 / 139 at 2048
+    if ((n & (n - 1)) == 0) return false;
+    if ((int64_t)n * c->d.ny * c->d.nz < 2500000) return true;  // 60 of the L2's 126 MB
     if (n % 7 == 0 || n % 11 == 0 || lb * per_sm <= 4) return true;
-    const bool in_l2 = (int64_t)n * c->d.ny * c->d.nz < 4000000;  // 3 x 32 of 126 MB
-    if (x.p.rmax <= 8) return (dr_rows(c) && lb <= 6) || (in_l2 && x.p.nst == 3);
-    return c->fx.nrad >= 5 && (per_sm == 2 || in_l2);
+    return x.p.rmax <= 8 ? dr_rows(c) && lb <= 6 : c->fx.nrad >= 5 && per_sm == 2;
   }
 
   // mode 0: divergence of q; 1: stored RHSLLPHI; 2: residual buffer

@@ -392,9 +392,8 @@ def test_substep_calls_beside_a_capture_of_the_caller(mode):
 @pytest.mark.parametrize("nx", [28, 44, 54, 60, 66, 70, 84, 90, 98, 126, 144, 150, 162, 176, 210, 216, 242, 264, 288, 300, 324, 330, 350,
                                 360, 384, 432, 450, 462, 486, 588, 630])
 def test_x_transform_lengths_on_more_lines(nx):
-    """The x transforms over their radices on enough lines for the register-
-    blocked forward form, with an odd row count; the short list of
-    test_x_transform_lengths takes the staged one at most lengths."""
+    """The x transforms over their radices on more lines than a block holds,
+    with an odd row count."""
     g, o = pair(nx, 11, 240, seed=4)
     g.solverrk3_mom_tg(0)
     o.substep(0)
@@ -415,6 +414,16 @@ def test_transform_lengths_without_a_register_plan(dims):
 def test_z_transform_forms_by_grid(dims):
     """z lengths whose register lines come two to a block: staged on few
     blocks, register-blocked on many."""
+    g, o = pair(*dims, seed=4)
+    g.solverrk3_mom_tg(0)
+    o.substep(0)
+    compare(g, o, tag=str(dims))
+
+
+@pytest.mark.parametrize("dims", [(48, 217, 250), (96, 113, 240), (100, 105, 252), (240, 61, 176), (360, 40, 180), (640, 20, 200)])
+def test_staged_x_transform_of_larger_grids(dims):
+    """Lengths that are not powers of two on grids whose inputs exceed half the
+    L2: the staged forward x transform, with full and ragged row blocks."""
     g, o = pair(*dims, seed=4)
     g.solverrk3_mom_tg(0)
     o.substep(0)
