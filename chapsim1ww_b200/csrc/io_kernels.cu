@@ -1526,13 +1526,16 @@ int io_np_mom(chapsim_ctx *c, int ns, bool mass_parts);
 //   84x33x50 (195 blocks of 4)     17 - 21 - 23 - 33 /  7.7 -  8.5 -  9.9 - 12.3
 //   192x55x44 (462)                29 - 29 - 29 - 37 / 25.0 - 23.2 - 23.0 - 25.6
 //   160x96x50 (780)                45 - 45 - 43 - 55 / 38.1 - 36.4 - 35.5 - 34.1
+//   264x80x66 (1530)               82 - 76 - 77 - 78 / 68.4 - 64.8 - 63.4 - 62.2
 //   192x77x176 (2640)         128 - 119 - 119 - 126 / 114.8 - 108.4 - 106.8 - 104.8
 //   384x192x192 (13824)       622 - 552 - 554 - 554 / 612.2 - 573.3 - 559.7 - 551.6
 static int eng_march(const chapsim_ctx *c, dim3 grid) {
   if (!c->use_tma_io || c->cfg.precision == CHAPSIM_MIXED) return 0;
   const int64_t blocks4 = (int64_t)grid.x * grid.y * ((c->d.nz + 3) / 4);
   if (2 * blocks4 < 3 * c->nsm) return 0;
-  return blocks4 < 4 * c->nsm ? 4 : (blocks4 < 40 * c->nsm ? 8 : 16);
+  if (blocks4 < 4 * c->nsm) return 4;
+  // 16 planes: at most one wave of three blocks a multiprocessor, or many
+  return blocks4 < 8 * c->nsm || (blocks4 > 12 * c->nsm && blocks4 < 40 * c->nsm) ? 8 : 16;
 }
 
 int io_eng(chapsim_ctx *c, int ns) {
