@@ -196,3 +196,42 @@ def test_energy_substep_properties_are_the_models_at_its_enthalpy(table, engine,
     for n, v in got.items():
         ref = g.get_field(n)[:, 1:-1, :]
         assert relerr(v, ref) <= (1e-6 if far else 1e-4), n
+
+
+@pytest.mark.parametrize("dims", [(20, 6, 12), (40, 18, 24), (96, 46, 64)], ids=lambda d: "x".join(map(str, d)))
+def test_short_steps_take_the_expansion(table, engine, dims):
+    """Steps far below the expansion's limit (1e-3 of the half range; here
+    dt |u| |dh/dx| and the wall flux give 1e-4 and less) evaluate no tile of
+    the model a second time."""
+    from chapsim1ww_b200 import IOChannel, _lib
+    g = IOChannel(*dims, table=table, dt=1e-4)
+    g.set_props_mode(_lib.PROPS_MLP, engine)
+    g.random_fl_theml_fld_io(3, 0.1)
+    h = g.get_field("h")
+    z, y, x = np.meshgrid(*(np.linspace(0, 2 * np.pi, n, endpoint=False) for n in h.shape), indexing="ij")
+    h[:, 1:-1, :] = (0.3 + 0.2 * np.sin(x) * np.cos(y) * np.cos(z))[:, 1:-1, :]
+    g.set_field("h", h)
+    g.therm_prop_update(mode=1)
+    g.set_field("rhoh", g.get_field("rho") * h)
+    before = g.model_again_tiles()
+    g.solverrk3_eng_io(1)
+    assert g.model_again_tiles() == before
+
+
+def test_substep_calls_follow_the_property_mode(table, engine):
+    """Substep calls captured with one property kernel, then with the other:
+    bitwise as graph steps, whose captures a change of the mode drops too."""
+    from chapsim1ww_b200 import IOChannel, _lib
+    a, b = IOChannel(40, 18, 24, table=table), IOChannel(40, 18, 24, table=table)
+    for x in (a, b):
+        x.random_fl_theml_fld_io(7, 0.1)
+    for mode in (_lib.PROPS_MLP, _lib.PROPS_TABLE, _lib.PROPS_MLP):
+        for x in (a, b):
+            x.set_props_mode(mode, engine)
+        for _ in range(12):
+            for ns in (1, 2, 3):
+                a.solverrk3_eng_io(ns)
+                a.solverrk3_mom_io(ns)
+        b.step(12)
+        for f in FLOW + THERMAL:
+            assert np.array_equal(a.get_field(f), b.get_field(f)), (mode, f)
