@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(SI_BX *SI_BY, 4) k_io_rhs_si(TGDev d, IODev io
 // kernels above read up to fourteen arrays from global memory, 60 loads per
 // cell and component, and wait for them (DRAM 17 %): 3.15 ms for the three at
 // 384x192x192 with the energy equation, 1.00 ms here (its bytes: 0.37 ms;
-// shared-memory pipe 62 %, FP64 pipe 31 % busy).
+// at 192x96x192 L1 and shared memory 67 %, FP64 pipe 34 % busy).
 constexpr int ST_BXW = 36, ST_BYW = 10, ST_PLANE = ST_BXW * ST_BYW, ST_PST = 368;
 constexpr int S_U = 0, S_V = 1, S_W = 2, S_GX = 3, S_GY = 4, S_GZ = 5, S_P = 6, S_MU = 7, S_M = 8, S_R = 9;
 constexpr int st_fields(bool th) { return th ? 12 : 7; }
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(256) k_si_x(TGDev d, IODev io, double coe1, do
 // The y solve ends with G* = G + dG in the other G buffer from row N2I.
 // Four blocks per SM (64 registers, a few spilled words) with 8 lines each at
 // n = 192: the blocks' stage / solve / store phases overlap better than two
-// blocks of 16 lines.  Bound by instruction issue (55-60 %), so the staging
+// blocks of 16 lines.  Bound by instruction issue (47-56 %), so the staging
 // loops carry no divisions (1 / RHO_STG once per cell in k_si_stg, slots by
 // SlotWalk) and no branches (wall rows apart), and the reduction ends early:
 // x / z / y lines of one component at 384x192x192 260 / 335 / 560 -> 169 / 203

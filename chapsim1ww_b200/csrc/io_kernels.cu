@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(IO_BX *IO_BY, 6) k_io_eng_rhs(TGDev d, IODev i
 // ENTHALPY_UPDATE, THERM_PROP_UPDATE.  A look-up outside the table leaves the
 // value unchanged and is counted (the reference STOPs).
 // What bounds it is the L1 data pipe (87 % busy at 225 wavefronts per warp,
-// most of them the table gathers; DRAM 35 %): 0.574 -> 0.386 ms at
+// most of them the table gathers; DRAM 24 %): 0.574 -> 0.386 ms at
 // 384x192x192 with enthalpies varying from cell to cell, against 0.19 ms for
 // its bytes, since the look-ups read pair arrays instead of interval records
 // and the second look-up reuses the first one's interval.  Five blocks per
